@@ -1124,7 +1124,7 @@ extern "C" int pulpnn_linear_out_32_static_scratch(const uint8_t *pInBuffer, con
     return c.err;
   }
 
-  TcParams g;
+  TcParams g = {};
   g.M = n_vectors; g.N = num_o_neurons; g.K = dim_vec;
   g.epi = p.epi;
   g.conv = 0; g.tw_log2 = 7; g.tiles_x = g.tiles_y = 1; g.chunks_per_tap = 1;
