@@ -261,12 +261,33 @@ bool launch_dw_mode(Context &c, const DepthwiseProblem &p)
 
 }  // namespace
 
+// The plane-staging kernel has the shortest start, the TMA kernels and the one that keeps its rows in registers the
+// higher rate. Where the lines lie (bytes read and written; us planes / other kernel):
+//  HWC, TMA:   1x28x28x256 0.4 MB 2.4 / 5.4, 8x28x28x256 3.2 MB 5.0 / 5.5, 16x28x28x256 6.4 MB 7.0 / 5.5 -- wide images;
+//              8x14x14x512 1.6 MB 4.0 / 4.2, 16x14x14x512 3.2 MB 5.1 / 4.2; 1x7x7x1024 0.1 MB 2.3 / 2.9, 8x7x7x1024
+//              0.8 MB 3.3 / 2.9: the smaller the image, the shorter the TMA kernel's strips
+//  HWC, registers: 8x56x56x100 5.0 MB 7.3 / 8.3, 16x56x56x100 10 MB 11.3 / 9.6; stride 2: 6.3 MB 8.1 / 11.8, 12.5 MB 13.0 / 11.8
+//  CHW, TMA:   16x32x32x128 4.2 MB 6.2 / 7.3, 8x112x112x32 6.4 MB 8.2 / 7.8
+static bool planes_first(const DepthwiseProblem &p, bool tma)
+{
+  const long long bytes = (long long)p.B * p.C * ((long long)p.H * p.W + (long long)p.Ho * p.Wo);
+  long long kb;
+  if (!p.in_is_hwc) kb = 4500;
+  else if (tma)     kb = p.Wo >= 28 ? 3300 : (p.Wo >= 14 ? 1700 : 400);
+  else              kb = p.sx == 1 ? 6000 : 9000;
+  return bytes <= kb * 1000;
+}
+
 bool launch_depthwise(Context &c, const DepthwiseProblem &p)
 {
-  if (!c.opt_force_generic && depthwise_hwc3x3_tma_supported(p)) return launch_depthwise_hwc3x3_tma(c, p);
-  if (!c.opt_force_generic && depthwise_hwc3x3_supported(p)) return launch_depthwise_hwc3x3(c, p);
-  if (!c.opt_force_generic && depthwise_chw3x3_tma_supported(p)) return launch_depthwise_chw3x3_tma(c, p);
-  if (!c.opt_force_generic && depthwise_chw3x3_supported(p)) return launch_depthwise_chw3x3(c, p);
+  if (!c.opt_force_generic) {
+    const bool planes = depthwise_planes_supported(p);
+    const bool tma = p.in_is_hwc ? depthwise_hwc3x3_tma_supported(p) : depthwise_chw3x3_tma_supported(p);
+    if (tma && !(planes && planes_first(p, true)))
+      return p.in_is_hwc ? launch_depthwise_hwc3x3_tma(c, p) : launch_depthwise_chw3x3_tma(c, p);
+    if (depthwise_hwc3x3_supported(p) && !(planes && planes_first(p, false))) return launch_depthwise_hwc3x3(c, p);
+    if (planes) return launch_depthwise_planes(c, p);
+  }
   switch (p.epi.mode) {
     case EPI_NONE: return launch_dw_mode<EPI_NONE>(c, p);
     case EPI_MULT: return launch_dw_mode<EPI_MULT>(c, p);

@@ -1,0 +1,307 @@
+// depthwise_planes.cu -- 3x3 and 5x5 depthwise convolution, stride 1 or 2, of ANY channel count, row
+// length and alignment, from HWC or CHW input (arithmetic of 32bit/src/pulp_nn_depthwise_generic.c:133-180).
+//
+// A CTA takes one image, a group of 32 (16) channels and a band of output rows. It stages the input rows
+// of the band in shared memory as one PLANE per channel, [channel][row][x + padding_left], zeros outside
+// the image: HWC input through 4x4 byte transposes (four pixels x four channels), CHW input as it lies.
+// A lane is a channel, so a warp stores runs of 32 bytes of the HWC output and an odd pitch in words
+// keeps the lanes on different banks. A lane computes four adjacent output columns of R rows: their
+// windows lie in two (stride 1) or three (stride 2) aligned words of a plane row, and a filter row costs
+// one or two dp4a per output against copies of its taps shifted to the byte the window starts at -- no
+// unpacking and no funnel shifts. Each plane row is read once for the R rows it feeds.
+//
+// What bounds it: instruction issue -- a warp of 5x5 outputs costs some 25 instructions in the dp4a and
+// the requantised byte stores, about as many again to stage its share of the input (halo included) and to
+// set the CTA up. Measured (us, graph replay, before / after): 28x28x120 5x5 HWC at batch 32 39.3 / 10.9, the
+// same from CHW 97.8 / 11.3, 14x14x475 5x5 stride 2 at batch 20 15.9 / 6.1, 56x56x61 3x3 at batch 8 25.5 /
+// 5.7, 30x30x64 3x3 CHW at batch 64 70.9 / 8.9.
+#include "internal.cuh"
+#include "unaligned16.cuh"
+
+namespace pulpnn {
+
+namespace {
+
+constexpr int DT = 256;
+
+struct PlanesParams {
+  DepthwiseProblem p;
+  int groups, bands, band;      // channel groups, bands of `band` output rows (a multiple of R)
+  int rows_in, row_pitch;       // staged rows, bytes of a plane row
+  int plane;                    // bytes of a plane, an odd number of words
+  int words;                    // HWC: channels in whole aligned words
+  int quads;                    // groups of four output columns
+  FastDiv by_qw, by_per, by_quads;   // words (CHW: 16-byte pieces) of a plane row, of a plane; quads
+};
+
+__device__ __forceinline__ unsigned prmt_b(unsigned a, unsigned b, unsigned sel)
+{
+  unsigned d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
+}
+
+template <int MODE, int K, int S, int CG>
+__global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_constant__ PlanesParams g)
+{
+  constexpr int R = S == 1 ? 4 : 2;                         // output rows of a lane
+  constexpr int NW = ((3 * S + K - 1) >> 2) + 1;            // plane words its four columns touch
+  constexpr int NV = 4 / S;                                 // window starts modulo a word
+  extern __shared__ __align__(16) uint8_t planes[];
+  const DepthwiseProblem &p = g.p;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned blk = blockIdx.x;
+  const int grp = (int)(blk % (unsigned)g.groups); blk /= (unsigned)g.groups;
+  const int band = (int)(blk % (unsigned)g.bands);
+  const int b = (int)(blk / (unsigned)g.bands);
+  const int c0 = grp * CG, nch = min(CG, p.C - c0);
+  const int oy0 = band * g.band;
+  const int iy0 = oy0 * S - p.pt;
+  const int qw = g.row_pitch >> 2;                          // words of a plane row
+
+  pdl_wait();
+  pdl_launch_dependents();
+
+  // ---- stage the planes -----------------------------------------------------------------------
+  if (p.in_is_hwc) {
+    constexpr int CQ = CG / 4;
+    const uint8_t *img = p.in + (size_t)b * p.H * p.W * p.C + c0;
+    const int items = g.rows_in * qw;                       // words of four pixels, the thread's four channels
+    const int cq = tid % CQ, left = nch - 4 * cq;           // channels of this word that exist
+    constexpr int STEP = DT / CQ;
+    constexpr int U = 2;                                    // items of a thread in flight
+    for (int it0 = tid / CQ; it0 < items; it0 += U * STEP) {
+      unsigned v[U][4];
+      int dst[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int it = it0 + u * STEP;
+        const int row = g.by_qw.div(it), q = it - row * qw;
+        const int iy = iy0 + row;
+        const bool ok = it < items && (unsigned)iy < (unsigned)p.H && left > 0;
+        const int ix = 4 * q - p.pl;
+        const uint8_t *src = img + ((size_t)(ok ? iy : 0) * p.W + ix) * p.C + 4 * cq;
+        dst[u] = it < items ? 4 * cq * g.plane + row * g.row_pitch + 4 * q : -1;
+        if (g.words) {
+#pragma unroll
+          for (int i = 0; i < 4; i++) v[u][i] = ldg4_if(src + (size_t)i * p.C, ok && (unsigned)(ix + i) < (unsigned)p.W);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const bool in = ok && (unsigned)(ix + i) < (unsigned)p.W;
+            v[u][i] = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) v[u][i] |= ldg1_if(src + (size_t)i * p.C + k, in && k < left) << (8 * k);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (dst[u] < 0) continue;
+        const unsigned a = prmt_b(v[u][0], v[u][1], 0x5140), bb = prmt_b(v[u][0], v[u][1], 0x7362);
+        const unsigned cc = prmt_b(v[u][2], v[u][3], 0x5140), d = prmt_b(v[u][2], v[u][3], 0x7362);
+        uint8_t *to = planes + dst[u];
+        *reinterpret_cast<unsigned *>(to) = prmt_b(a, cc, 0x5410);
+        *reinterpret_cast<unsigned *>(to + g.plane) = prmt_b(a, cc, 0x7632);
+        *reinterpret_cast<unsigned *>(to + 2 * g.plane) = prmt_b(bb, d, 0x5410);
+        *reinterpret_cast<unsigned *>(to + 3 * g.plane) = prmt_b(bb, d, 0x7632);
+      }
+    }
+  } else {
+    // offsets from the group's first byte, with up to 64 bytes of the tensor on either side: a piece is read as two
+    // aligned blocks of 16, which only at the very ends of the tensor are not its own
+    const size_t off = ((size_t)b * p.C + c0) * p.H * p.W, all = (size_t)p.B * p.C * p.H * p.W;
+    const int own = nch * p.H * p.W;
+    const int before = (int)min(off, (size_t)64), after = (int)min(all - off - (size_t)own, (size_t)64);
+    const Bytes in(p.in + off - before, before + own + after);
+    const int first = in.start + before;
+    const int pw = g.row_pitch >> 4, per = g.rows_in * pw, items = per * nch;   // 16-byte pieces
+    constexpr int U = 2;
+    for (int it0 = tid; it0 < items; it0 += U * DT) {
+      Chunk t[U];
+      int from[U], to[U], dst[U];                           // bytes [from, to) of the piece lie inside the image
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int it = it0 + u * DT;
+        const int ch = g.by_per.div(it), rq = it - ch * per;
+        const int row = g.by_qw.div(rq), q = rq - row * pw;
+        const int iy = iy0 + row, ix = 16 * q - p.pl;
+        from[u] = max(-ix, 0);
+        to[u] = it < items && (unsigned)iy < (unsigned)p.H && from[u] < 16 ? min(p.W - ix, 16) : 0;
+        t[u].fetch(in, first + (ch * p.H + iy) * p.W + ix, to[u] > 0);
+        dst[u] = it < items ? ch * g.plane + row * g.row_pitch + 16 * q : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (dst[u] < 0) continue;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (to[u] > 0) {
+          v = t[u].get(in);
+          if (from[u] > 0 || to[u] < 16) mask16(v, from[u], to[u]);
+        }
+        unsigned *d = reinterpret_cast<unsigned *>(planes + dst[u]);
+        d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+      }
+    }
+  }
+
+  // ---- this lane's channel: shifted copies of its filter rows, requantisation parameters -----------
+  const int cl = lane % CG, sub = lane / CG;
+  const int c = c0 + min(cl, nch - 1);
+  unsigned wv[K][NV][2];
+#pragma unroll
+  for (int fy = 0; fy < K; fy++) {
+    unsigned long long t = 0;
+#pragma unroll
+    for (int fx = 0; fx < K; fx++)
+      t |= (unsigned long long)(uint8_t)__ldg(p.w + ((size_t)c * K + fy) * K + fx) << (8 * fx);
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      wv[fy][v][0] = (unsigned)(t << (8 * v * S));
+      wv[fy][v][1] = (unsigned)((t << (8 * v * S)) >> 32);
+    }
+  }
+  const Epilogue &e = p.epi;
+  long long kk = 0, ll = 0;
+  if (MODE == EPI_BN32) {
+    kk = __ldg(reinterpret_cast<const int *>(e.k) + c);
+    ll = __ldg(reinterpret_cast<const int *>(e.lambda) + c);
+  } else if (MODE == EPI_BN64) {
+    kk = __ldg(reinterpret_cast<const long long *>(e.k) + c);
+    ll = __ldg(reinterpret_cast<const long long *>(e.lambda) + c);
+  }
+  const int bias = e.bias ? (int)__ldg(reinterpret_cast<const int8_t *>(e.bias) + c) : 0;
+  __syncthreads();
+
+  // ---- compute: a unit is four columns x R rows of the warp's channels ------------------------------
+  const int rows = min(g.band, p.Ho - oy0);
+  const int units = ((rows + R - 1) / R) * g.quads;
+  const uint8_t *mine = planes + (size_t)cl * g.plane;
+  for (int u = warp * (32 / CG) + sub; u < units; u += (DT / 32) * (32 / CG)) {
+    const int rb = g.by_quads.div(u), xq = u - rb * g.quads;
+    int acc[R][4];
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) acc[r][i] = bias;
+    const uint8_t *at = mine + (rb * R * S) * g.row_pitch + xq * 4 * S;
+#pragma unroll
+    for (int ir = 0; ir < S * (R - 1) + K; ir++) {
+      unsigned w[NW];
+#pragma unroll
+      for (int j = 0; j < NW; j++) w[j] = *reinterpret_cast<const unsigned *>(at + ir * g.row_pitch + 4 * j);
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const int fy = ir - S * r;
+        if (fy < 0 || fy >= K) continue;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int off = (i * S) & 3, j = (i * S) >> 2;
+          acc[r][i] = dp4a_us(w[j], (int)wv[fy][off / S][0], acc[r][i]);
+          if (off + K > 4) acc[r][i] = dp4a_us(w[j + 1 < NW ? j + 1 : j], (int)wv[fy][off / S][1], acc[r][i]);
+        }
+      }
+    }
+    if (cl < nch) {
+      const int oy = oy0 + rb * R, ox = xq * 4;
+      uint8_t *o = p.out + (((size_t)b * p.Ho + oy) * p.Wo + ox) * p.C + c;
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        if (oy + r >= p.Ho) break;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          if (ox + i < p.Wo) o[((size_t)r * p.Wo + i) * p.C] = (uint8_t)requant_kl<MODE>(acc[r][i], kk, ll, e.out_mult, e.shift);
+      }
+    }
+  }
+}
+
+template <int MODE, int K, int S, int CG>
+bool launch_planes(Context &c, const PlanesParams &g, int smem)
+{
+  auto kern = depthwise_planes_kernel<MODE, K, S, CG>;
+  static PerDeviceInt attr_set;
+  if (!attr_set.get(c.device)) {
+    if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), "cudaFuncSetAttribute(depthwise_planes)"))
+      return false;
+    attr_set.set(c.device, 1);
+  }
+  const cudaError_t le = launch_pdl(kern, dim3((unsigned)(g.groups * g.bands * g.p.B)), dim3(DT), (size_t)smem, c.stream, g);
+  count_launch("depthwise_planes_kernel");
+  return cuda_ok(le, "depthwise_planes launch") && cuda_ok(cudaGetLastError(), "depthwise_planes launch");
+}
+
+template <int MODE, int CG>
+bool launch_planes_ks(Context &c, const PlanesParams &g, int smem)
+{
+  if (g.p.kx == 3) return g.p.sx == 1 ? launch_planes<MODE, 3, 1, CG>(c, g, smem) : launch_planes<MODE, 3, 2, CG>(c, g, smem);
+  return g.p.sx == 1 ? launch_planes<MODE, 5, 1, CG>(c, g, smem) : launch_planes<MODE, 5, 2, CG>(c, g, smem);
+}
+
+template <int MODE>
+bool launch_planes_mode(Context &c, const PlanesParams &g, int cg, int smem)
+{
+  return cg == 16 ? launch_planes_ks<MODE, 16>(c, g, smem) : launch_planes_ks<MODE, 32>(c, g, smem);
+}
+
+// lays the work out; false when not even one band of R rows fits shared memory or the grid is too large
+bool configure(const DepthwiseProblem &p, int sms, PlanesParams &g, int &cg, int &smem)
+{
+  const int S = p.sx, K = p.kx, R = S == 1 ? 4 : 2;
+  g.p = p;
+  cg = p.C <= 16 ? 16 : 32;
+  g.groups = (p.C + cg - 1) / cg;
+  g.quads = (p.Wo + 3) / 4;
+  long long pitch = (long long)(g.quads - 1) * 4 * S + 4 * (((3 * S + K - 1) >> 2) + 1);
+  if (!p.in_is_hwc) pitch = (pitch + 15) & ~15LL;           // rows are staged in 16-byte pieces
+  g.words = p.C % 4 == 0 && (reinterpret_cast<uintptr_t>(p.in) & 3) == 0;
+  auto plane_of = [&](int band) {
+    long long w = ((long long)(band - 1) * S + K) * (pitch / 4);
+    return (w | 1) * 4;
+  };
+  // whole images while they fit 48 KB (four CTAs of an SM), shorter bands until the GPU is full
+  const int rb = (p.Ho + R - 1) / R;
+  int blocks = rb;
+  while (blocks > 1 && (plane_of(blocks * R) * cg > 48 * 1024 || (long long)p.B * g.groups * ((rb + blocks - 1) / blocks) < 2LL * sms))
+    blocks = (blocks + 1) / 2;
+  g.band = blocks * R;
+  if (plane_of(g.band) * cg > 200 * 1024) return false;
+  // 32-bit offsets inside a group of channels, the rows above and below its image included
+  if (((long long)cg * p.H + p.pt + g.band * S + K) * p.W > 0x7fff0000LL) return false;
+  g.bands = (p.Ho + g.band - 1) / g.band;
+  if ((long long)g.groups * g.bands * p.B > 0x7fffffffLL) return false;
+  g.row_pitch = (int)pitch;
+  g.rows_in = (g.band - 1) * S + K;
+  g.plane = (int)plane_of(g.band);
+  smem = g.plane * cg;
+  const int piece = p.in_is_hwc ? 4 : 16;
+  g.by_qw.set((unsigned)(g.row_pitch / piece));
+  g.by_per.set((unsigned)(g.rows_in * (g.row_pitch / piece)));
+  g.by_quads.set((unsigned)g.quads);
+  return true;
+}
+
+}  // namespace
+
+bool depthwise_planes_supported(const DepthwiseProblem &p)
+{
+  if (p.kx != p.ky || (p.kx != 3 && p.kx != 5) || p.sx != p.sy || (p.sx != 1 && p.sx != 2)) return false;
+  PlanesParams g = {};
+  int cg, smem;
+  return configure(p, 148, g, cg, smem);
+}
+
+bool launch_depthwise_planes(Context &c, const DepthwiseProblem &p)
+{
+  PlanesParams g = {};
+  int cg, smem;
+  if (!configure(p, c.sm_count > 0 ? c.sm_count : 148, g, cg, smem)) return false;
+  switch (p.epi.mode) {
+    case EPI_NONE: return launch_planes_mode<EPI_NONE>(c, g, cg, smem);
+    case EPI_MULT: return launch_planes_mode<EPI_MULT>(c, g, cg, smem);
+    case EPI_BN32: return launch_planes_mode<EPI_BN32>(c, g, cg, smem);
+    default:       return launch_planes_mode<EPI_BN64>(c, g, cg, smem);
+  }
+}
+
+}  // namespace pulpnn

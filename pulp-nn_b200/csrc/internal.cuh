@@ -93,6 +93,24 @@ __device__ __forceinline__ int dp4a_us(unsigned a_u8x4, int b_s8x4, int c)
   return d;
 }
 
+// Division of 0 .. 2^31-1 by a constant of the launch: a multiply and a shift where the hardware's
+// integer division takes some 25 instructions (Granlund and Montgomery, division by invariant integers).
+struct FastDiv {
+  unsigned d, mul, shift;
+  void set(unsigned v)
+  {
+    d = v; mul = 0; shift = 0;
+    if (v <= 1) return;
+    unsigned l = 1;
+    while ((1ull << l) < v) l++;
+    mul = (unsigned)(((1ull << (31 + l)) + v - 1) / v);
+    shift = l - 1;
+  }
+#ifdef __CUDACC__
+  __device__ __forceinline__ int div(int n) const { return d == 1 ? n : (int)(__umulhi((unsigned)n, mul) >> shift); }
+#endif
+};
+
 // ---------------------------------------------------------------------------------------------
 // Problem descriptions handed from the entry points to the launchers (all pointers are device
 // pointers by then).
@@ -246,8 +264,9 @@ bool launch_dwpw_fused(Context &c, const DepthwiseProblem &dw, const ConvProblem
 // the 32 -> 64 channel pair with the depthwise layer on the tensor cores too (dwpw_tcdw.cu)
 bool dwpw_tcdw_supported(const DepthwiseProblem &dw, const ConvProblem &pw);
 bool launch_dwpw_tcdw(Context &c, const DepthwiseProblem &dw, const ConvProblem &pw);
-bool depthwise_chw3x3_supported(const DepthwiseProblem &p);
-bool launch_depthwise_chw3x3(Context &c, const DepthwiseProblem &p);
+// 3x3 / 5x5 at any channel count and alignment, HWC or CHW input, from planes in shared memory
+bool depthwise_planes_supported(const DepthwiseProblem &p);
+bool launch_depthwise_planes(Context &c, const DepthwiseProblem &p);
 int *ctx_status_word(Context &c);               // allocated on first use; nullptr on failure
 int static_scratch_status_take(Context &c);     // status of the no-allocation entry point (0: unused or fine)
 bool launch_maxpool(Context &c, const PoolProblem &p, uint8_t *clobber_in);
