@@ -7,6 +7,7 @@ the library is the address. Device memory is used in place; host memory is stage
 library itself. Errors recorded by the library are raised as ``PulpNNError``.
 """
 import ctypes as C
+import struct
 
 import numpy as np
 
@@ -102,12 +103,68 @@ def get_option(option):
     return _lib.load_library().pulpnn_get_option(int(option))
 
 
+# ---- calls with packed arguments (csrc/packed_calls.cu) ----------------------------------------
+# The common case of every entry point: arguments that struct packs as they are go over as one block of bytes.
+# Whatever it does not take (a value that the C type cuts, an object without an integer) goes argument by argument,
+# with the conversions and errors of ctypes.
+def _addr(x):
+    """Address of a buffer as an integer, 0 for None."""
+    if x is None:
+        return 0
+    try:
+        a = x.data_ptr()
+    except AttributeError:
+        return _ptr(x).value or 0
+    assert x.is_contiguous(), "buffers must be contiguous"
+    return a
+
+
+class _Packed:
+    """call(bits, ...) of one packed entry point; `through` names the entry it forwards to, if it serves several."""
+
+    def __init__(self, name, fmt, through=None):
+        self.name, self.pack, self.through, self.bound = name, struct.Struct(fmt).pack, through, {}
+
+    def bind(self, bits):
+        f = getattr(_lib.load_library(), "pulpnn_packed_" + self.name + _sfx(bits))
+        f.restype = C.c_int
+        if self.through is None:
+            f.argtypes = [C.c_char_p]
+            call = f
+        else:
+            # the library's functions are shared objects of ctypes: a prototype of our own leaves theirs alone
+            proto = C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_char_p)
+            fn = proto(C.cast(f, C.c_void_p).value)
+            entry = C.cast(_fn(self.through, bits), C.c_void_p)
+            call = lambda block: fn(entry, block)  # noqa: E731
+        self.bound[bits] = call
+        return call
+
+    def __call__(self, bits, *args):
+        """False when the arguments do not pack."""
+        try:
+            block = self.pack(*args)
+        except struct.error:
+            return False
+        call = self.bound.get(bits) or self.bind(bits)
+        if call(block):
+            _check()
+        return True
+
+
 # ---- kernel entry points ---------------------------------------------------------------------
 def _conv_like(name):
+    packed = _Packed("conv", "=7Q16H2i", name)
+
     def call(bits, pInBuffer, pIm2ColBuffer, bias, pOutBuffer, pWeight, k, lambda_, out_mult,
              out_shift, dim_in_x, dim_in_y, ch_in, dim_out_x, dim_out_y, ch_out, dim_kernel_x,
              dim_kernel_y, padding_y_top, padding_y_bottom, padding_x_left, padding_x_right,
              stride_x, stride_y, flag_relu, flag_batch_norm):
+        if packed(bits, _addr(pInBuffer), _addr(pIm2ColBuffer), _addr(bias), _addr(pOutBuffer), _addr(pWeight), _addr(k),
+                  _addr(lambda_), out_mult, out_shift, dim_in_x, dim_in_y, ch_in, dim_out_x, dim_out_y, ch_out,
+                  dim_kernel_x, dim_kernel_y, padding_y_top, padding_y_bottom, padding_x_left, padding_x_right, stride_x,
+                  stride_y, flag_relu, flag_batch_norm):
+            return
         _fn(name, bits)(_ptr(pInBuffer), _ptr(pIm2ColBuffer), _ptr(bias), _ptr(pOutBuffer),
                         _ptr(pWeight), _ptr(k), _ptr(lambda_), C.c_uint16(out_mult),
                         C.c_uint16(out_shift), C.c_uint16(dim_in_x), C.c_uint16(dim_in_y),
@@ -132,10 +189,17 @@ pulp_nn_pointwise_Co_parallel = _conv_like("pulp_nn_pointwise_Co_parallel")
 
 
 def _dw_like(name):
+    packed = _Packed("depthwise", "=8Q16H2b", name)
+
     def call(bits, Im_in, bufferC, bias, Im_out, wt, bufferB, k, lambda_, out_mult, out_shift,
              dim_im_in_x, dim_im_in_y, ch_im_in, dim_im_out_x, dim_im_out_y, ch_im_out,
              dim_kernel_x, dim_kernel_y, padding_y_top, padding_y_bottom, padding_x_left,
              padding_x_right, stride_x, stride_y, FLAG_RELU, FLAG_BATCH_NORM):
+        if packed(bits, _addr(Im_in), _addr(bufferC), _addr(bias), _addr(Im_out), _addr(wt), _addr(bufferB), _addr(k),
+                  _addr(lambda_), out_mult, out_shift, dim_im_in_x, dim_im_in_y, ch_im_in, dim_im_out_x, dim_im_out_y,
+                  ch_im_out, dim_kernel_x, dim_kernel_y, padding_y_top, padding_y_bottom, padding_x_left, padding_x_right,
+                  stride_x, stride_y, FLAG_RELU, FLAG_BATCH_NORM):
+            return
         _fn(name, bits)(_ptr(Im_in), _ptr(bufferC), _ptr(bias), _ptr(Im_out), _ptr(wt),
                         _ptr(bufferB), _ptr(k), _ptr(lambda_), C.c_uint16(out_mult),
                         C.c_uint16(out_shift), C.c_uint16(dim_im_in_x), C.c_uint16(dim_im_in_y),
@@ -177,8 +241,18 @@ def pulp_nn_matmul(bits, pWeight, pInBuffer, ch_out, num_col_im2col, out_shift, 
     return r
 
 
+_linear = _Packed("linear", "=6QHb2H2i")
+_linear_out_32 = _Packed("linear_out_32", "=4Q2H")
+_maxpool = _Packed("maxpool", "=2Q13H")
+_avgpool = _Packed("avgpool", "=2QqHq13Hi")
+_add = _Packed("add", "=3Q6H")
+
+
 def pulp_nn_linear(bits, pInBuffer, bias, pOutBuffer, pWeights, k, lambda_, out_mult, out_shift,
                    dim_vec, num_o_neurons, flag_relu, flag_batch_norm):
+    if _linear(bits, _addr(pInBuffer), _addr(bias), _addr(pOutBuffer), _addr(pWeights), _addr(k), _addr(lambda_), out_mult,
+               out_shift, dim_vec, num_o_neurons, flag_relu, flag_batch_norm):
+        return
     _fn("pulp_nn_linear", bits)(_ptr(pInBuffer), _ptr(bias), _ptr(pOutBuffer), _ptr(pWeights),
                                 _ptr(k), _ptr(lambda_), C.c_uint16(out_mult), C.c_int8(out_shift),
                                 C.c_uint16(dim_vec), C.c_uint16(num_o_neurons), C.c_int(flag_relu),
@@ -187,6 +261,8 @@ def pulp_nn_linear(bits, pInBuffer, bias, pOutBuffer, pWeights, k, lambda_, out_
 
 
 def pulp_nn_linear_out_32(bits, pInBuffer, bias, pOutBuffer, pWeights, dim_vec, num_o_neurons):
+    if _linear_out_32(bits, _addr(pInBuffer), _addr(bias), _addr(pOutBuffer), _addr(pWeights), dim_vec, num_o_neurons):
+        return
     _fn("pulp_nn_linear_out_32", bits)(_ptr(pInBuffer), _ptr(bias), _ptr(pOutBuffer),
                                        _ptr(pWeights), C.c_uint16(dim_vec),
                                        C.c_uint16(num_o_neurons))
@@ -203,6 +279,9 @@ def _geom(dim_im_in_x, dim_im_in_y, ch_im_in, dim_im_out_x, dim_im_out_y, dim_ke
 def pulp_nn_maxpool(bits, Im_in, Im_out, dim_im_in_x, dim_im_in_y, ch_im_in, dim_im_out_x,
                     dim_im_out_y, dim_kernel_x, dim_kernel_y, padding_t, padding_b, padding_l,
                     padding_r, stride_x, stride_y):
+    if _maxpool(bits, _addr(Im_in), _addr(Im_out), dim_im_in_x, dim_im_in_y, ch_im_in, dim_im_out_x, dim_im_out_y,
+                dim_kernel_x, dim_kernel_y, padding_t, padding_b, padding_l, padding_r, stride_x, stride_y):
+        return
     _fn("pulp_nn_maxpool", bits)(_ptr(Im_in), _ptr(Im_out),
                                  *_geom(dim_im_in_x, dim_im_in_y, ch_im_in, dim_im_out_x,
                                         dim_im_out_y, dim_kernel_x, dim_kernel_y, padding_t,
@@ -213,6 +292,10 @@ def pulp_nn_maxpool(bits, Im_in, Im_out, dim_im_in_x, dim_im_in_y, ch_im_in, dim
 def pulp_nn_avgpool(bits, Im_in, Im_out, lambda_, out_shift, out_add, dim_im_in_x, dim_im_in_y,
                     ch_im_in, dim_im_out_x, dim_im_out_y, dim_kernel_x, dim_kernel_y, padding_t,
                     padding_b, padding_l, padding_r, stride_x, stride_y, flag_requant):
+    if _avgpool(bits, _addr(Im_in), _addr(Im_out), int(lambda_), out_shift, int(out_add), dim_im_in_x, dim_im_in_y, ch_im_in,
+                dim_im_out_x, dim_im_out_y, dim_kernel_x, dim_kernel_y, padding_t, padding_b, padding_l, padding_r,
+                stride_x, stride_y, flag_requant):
+        return
     bn_t = C.c_int32 if bits == 32 else C.c_int64
     _fn("pulp_nn_avgpool", bits)(_ptr(Im_in), _ptr(Im_out), bn_t(int(lambda_)),
                                  C.c_uint16(out_shift), bn_t(int(out_add)),
@@ -225,6 +308,9 @@ def pulp_nn_avgpool(bits, Im_in, Im_out, lambda_, out_shift, out_add, dim_im_in_
 
 def pulp_nn_add(bits, Im_in_1, Im_in_2, Im_out, out_mult1, out_mult2, out_shift, dim_im_in_h,
                 dim_im_in_w, ch_im_in):
+    if _add(bits, _addr(Im_in_1), _addr(Im_in_2), _addr(Im_out), out_mult1, out_mult2, out_shift, dim_im_in_h, dim_im_in_w,
+            ch_im_in):
+        return
     _fn("pulp_nn_add", bits)(_ptr(Im_in_1), _ptr(Im_in_2), _ptr(Im_out), C.c_uint16(out_mult1),
                              C.c_uint16(out_mult2), C.c_uint16(out_shift),
                              C.c_uint16(dim_im_in_h), C.c_uint16(dim_im_in_w),
