@@ -108,6 +108,17 @@ int *ctx_status_word(Context &c)
   return c.status_word;
 }
 
+bool ctx_status_word_unless_capturing(Context &c, int **word)
+{
+  if (!c.status_word) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c.stream, &cap) != cudaSuccess) { cudaGetLastError(); cap = cudaStreamCaptureStatusActive; }
+    if (cap == cudaStreamCaptureStatusNone && !ctx_status_word(c)) return false;
+  }
+  *word = c.status_word;
+  return true;
+}
+
 // ---- staging ------------------------------------------------------------------------------
 static bool is_device_pointer(const void *p)
 {

@@ -28,6 +28,7 @@
 // 100 13.3 / 362 (79 before the reduction was shared in a cluster), 7x7x16 -> 16 3.8 / 7.3.
 #include "internal.cuh"
 #include "sm100_primitives.cuh"
+#include "split_epilogue.cuh"
 #include "unaligned16.cuh"
 
 namespace pulpnn {
@@ -54,81 +55,6 @@ struct GatherParams {
   int out_vec;             // store width in bytes: 16, 4 or 1
   int *status;
 };
-
-template <int MODE>
-__device__ __forceinline__ int requant_param(int a, int col, const long long *par_k, const long long *par_l, const Epilogue &e)
-{
-  const int *k32 = reinterpret_cast<const int *>(par_k), *l32 = reinterpret_cast<const int *>(par_l);
-  if (MODE == EPI_BN32) return (int)((unsigned)k32[col] * (unsigned)a + (unsigned)l32[col]) >> e.shift;
-  if (MODE == EPI_BN64)
-    return (int)((long long)((unsigned long long)par_k[col] * (unsigned long long)(long long)a + (unsigned long long)par_l[col]) >> e.shift);
-  if (MODE == EPI_MULT) return (int)(short)((int)((unsigned)e.out_mult * (unsigned)(a + l32[col])) >> e.shift);
-  return (a + l32[col]) >> e.shift;
-}
-
-// The CTAs of a cluster hold partial sums of the same tile: each puts its own into its shared memory,
-// takes an equal share of the rows, adds the others' through the cluster and finishes them. The sums
-// are integers, so their order does not matter.
-template <int MODE>
-__device__ __noinline__ void split_epilogue(const GatherParams &g, uint8_t *ring, uint32_t tmem, const long long *par_k,
-                                            const long long *par_l, int ks, int mt, int n0, int ncols, bool dead)
-{
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int pitch = g.bn + 4;                        // words; rows 16-byte aligned, an odd number of 16-byte pieces
-  const int quad = warp & 3, r = quad * 32 + lane;
-  if (!dead) {
-    for (int c0 = (warp >> 2) * 32; c0 < ncols; c0 += 64) {
-      uint32_t v[32];
-      tmem_ld_32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
-      tmem_wait_ld();
-      const uint32_t row = smem_u32(ring) + (uint32_t)((r * pitch + c0) * 4);
-#pragma unroll
-      for (int j = 0; j < 32; j += 4)
-        if (c0 + j < g.bn) sts128(row + 4 * j, v[j], v[j + 1], v[j + 2], v[j + 3]);
-    }
-  }
-  tc_fence_before();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  tc_fence_after();
-  const Epilogue &e = g.p.epi;
-  const int share = GBM / g.k_split, r0 = ks * share;
-  const int rows = min(share, g.M - mt * GBM - r0), per = (ncols + 3) >> 2;
-  if (!dead) {
-    for (int i = tid; i < rows * per; i += GT) {
-      const int rr = i / per, c = (i - rr * per) * 4;
-      const uint32_t mine = smem_u32(ring) + (uint32_t)(((r0 + rr) * pitch + c) * 4);
-      int s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-      for (int k = 0; k < g.k_split; k++) {
-        uint32_t a, x0, x1, x2, x3;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(mine), "r"(k));
-        asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x0), "=r"(x1), "=r"(x2), "=r"(x3) : "r"(a) : "memory");
-        s0 += (int)x0; s1 += (int)x1; s2 += (int)x2; s3 += (int)x3;
-      }
-      const size_t o = (size_t)(mt * GBM + r0 + rr) * g.p.Cout + n0 + c;
-      const int sum[4] = {s0, s1, s2, s3};
-      if (MODE == EPI_RAW32) {
-        int *out = reinterpret_cast<int *>(g.p.out) + o;
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-          if (c + j < ncols) out[j] = sum[j] + reinterpret_cast<const int *>(par_l)[c + j];
-      } else {
-        uint8_t *out = static_cast<uint8_t *>(g.p.out) + o;
-        int t[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) t[j] = requant_param<MODE>(sum[j], c + j, par_k, par_l, e);
-        const unsigned w = pack4_sat_u8(t[0], t[1], t[2], t[3]);
-        if (c + 4 <= ncols && (reinterpret_cast<uintptr_t>(out) & 3) == 0) *reinterpret_cast<unsigned *>(out) = w;
-        else {
-#pragma unroll
-          for (int j = 0; j < 4; j++)
-            if (c + j < ncols) out[j] = (uint8_t)(w >> (8 * j));
-        }
-      }
-    }
-  }
-  // nobody's sums are overwritten, and no CTA leaves, before all have read them
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 // ALIGNED: ch_in a multiple of 16 and 16-byte aligned operands, so that every chunk is one aligned load of one pixel
 // W_RES: the CTA's rows of W stay in shared memory
@@ -174,27 +100,8 @@ __global__ void __launch_bounds__(GT, 2) conv_gather_tc_kernel(const __grid_cons
   pdl_wait();
   pdl_launch_dependents();
 
-  // per-channel parameters; the bias is folded into lambda: k*(acc+b)+lambda == k*acc + (k*b+lambda) in
-  // wrap-around arithmetic
+  stage_channel_params<MODE>(p.epi, n0, ncols, par_k, par_l, tid, GT);
   const Epilogue &e = p.epi;
-  for (int i = tid; i < ncols; i += GT) {
-    const int n = n0 + i;
-    if (MODE == EPI_BN32) {
-      const int k = __ldg(reinterpret_cast<const int *>(e.k) + n), l = __ldg(reinterpret_cast<const int *>(e.lambda) + n);
-      const int b = e.bias ? (int)__ldg(reinterpret_cast<const int8_t *>(e.bias) + n) : 0;
-      reinterpret_cast<int *>(par_k)[i] = k;
-      reinterpret_cast<int *>(par_l)[i] = (int)((unsigned)k * (unsigned)b + (unsigned)l);
-    } else if (MODE == EPI_BN64) {
-      const long long k = __ldg(reinterpret_cast<const long long *>(e.k) + n), l = __ldg(reinterpret_cast<const long long *>(e.lambda) + n);
-      const long long b = e.bias ? (long long)__ldg(reinterpret_cast<const int8_t *>(e.bias) + n) : 0;
-      par_k[i] = k;
-      par_l[i] = (long long)((unsigned long long)k * (unsigned long long)b + (unsigned long long)l);
-    } else if (MODE == EPI_RAW32) {
-      reinterpret_cast<int *>(par_l)[i] = e.bias ? __ldg(reinterpret_cast<const int *>(e.bias) + n) : 0;
-    } else {
-      reinterpret_cast<int *>(par_l)[i] = e.bias ? (int)__ldg(reinterpret_cast<const int8_t *>(e.bias) + n) : 0;
-    }
-  }
 
   const int ck = tid & 7, row0 = tid >> 3;           // this thread's chunk of a slab, its first row
   const Bytes wt(p.w, p.Cout * g.K), at(p.in, p.B * p.H * p.W * p.Cin);
@@ -358,7 +265,9 @@ __global__ void __launch_bounds__(GT, 2) conv_gather_tc_kernel(const __grid_cons
     tc_fence_after();
 
     if (g.k_split > 1) {
-      split_epilogue<MODE>(g, ring, tmem, par_k, par_l, ks, mt, n0, ncols, dead);
+      const int m0 = mt * GBM;
+      split_epilogue<MODE>(p.epi, p.out, p.Cout, bn, g.k_split, ks, n0, ncols, ring, tmem, par_k, par_l, dead,
+                           [&](int r) { return m0 + r < g.M ? (long long)(m0 + r) : -1ll; });
       continue;
     }
 
@@ -584,13 +493,7 @@ bool launch_conv_gather_tc(Context &c, const ConvProblem &p)
   g.stages = stages;
   const int smem = (int)(w_res ? w_all : 0) + stages * stage + 1024;
 
-  if (!c.status_word) {
-    // nothing may be allocated while the stream is being captured; without the word a wait still ends
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c.stream, &cap) != cudaSuccess) { cudaGetLastError(); cap = cudaStreamCaptureStatusActive; }
-    if (cap == cudaStreamCaptureStatusNone && !ctx_status_word(c)) return false;
-  }
-  g.status = c.status_word;
+  if (!ctx_status_word_unless_capturing(c, &g.status)) return false;
 
   const int lanes = g.n_tiles * g.k_split;             // CTAs that work on one row of tiles
   int per = 2 * sms / lanes;

@@ -417,9 +417,51 @@ void add_entry(uint8_t *a, uint8_t *b, uint8_t *out, int m1, int m2, int out_shi
 }  // namespace
 
 // contraction dispatch: tensor cores where the shape allows, CUDA cores otherwise
+// Which kernel takes a GEMM of few tiles: the dp4a one while a CTA's eight neurons see few rows; igemm_split where a
+// cluster shares the reduction; the gathering kernel for narrow channel slabs, whose TMA boxes of 32 or 64 bytes a
+// row cost more than gathering them; igemm_tc otherwise. Measured (us, igemm_tc / gather / split, dp4a):
+//   196 x 512 -> 512     5.4 / 5.3 / 4.6, 13.7      196 x 256 -> 512   3.8 / 4.0 / 4.7, 13.9     392 x 512 -> 512  5.5 / 6.9 / 5.7
+//   49 x 512 -> 1024     5.2 / 5.1 / 4.6,  5.0      49 x 1024 -> 1024  9.6 / 5.6 / 5.2,  6.9     196 x 1024 -> 1024  14.2 / 7.3 / 5.7
+//   1 x 1024 -> 1000     8.2 / 5.2 / 4.9,  2.2      37 x 1024 -> 1000  9.2 / 5.6 / 5.1,  4.8     128 x 1024 -> 1000  13.2 / 5.8 / 5.2, 11.8
+//   1 x 4096 -> 4096     9.9 / 18  / 9.4,  5.6      16 x 4096 -> 4096  10.4 / 19 / 9.8, 13.9     128 x 4096 -> 4096  16.5 / 20 / 10.3, 87
+//   256 x 4096 -> 4096  17.4 / 33  / 13.0           512 x 4096 -> 4096 17.5 / 34 / 19.4          784 x 1024 -> 1024  7.7 / 9.8 / 9.2
+//   3x3, one image: 32x32x32 -> 64 8.1 / 4.4 / 7.7, 14x14x64 -> 64 8.1 / 5.4 / 7.5, 28x28x128 -> 128 10.4 / 6.6 / 6.8,
+//   7x7x512 -> 512 10.1 / 8.5 / 7.1; 14x14x256 -> 256 at batch 8 14.3 / 11.1 / 9.1, 28x28x128 -> 128 at batch 4 7.4 / 9.1 / 8.2
+enum class FewTiles { none, rows, gather, split };
+static FewTiles few_tiles_form(const Context &c, const ConvProblem &p)
+{
+  if (c.opt_force_generic || c.opt_split_k != 0 || !igemm_tc_supported(c, p)) return FewTiles::none;
+  const long long M = (long long)p.B * p.Ho * p.Wo;
+  const int sms = c.sm_count > 0 ? c.sm_count : 148;
+  const bool plain = p.ky * p.kx == 1 && p.H == p.Ho && p.W == p.Wo;
+  bool few;
+  const int tiles = igemm_tc_tiles(c, p, &few);
+  if (!plain) {
+    if (tiles > sms || !few) return FewTiles::none;
+    return (p.Cin % 128 == 0 && p.Cin >= 256) || !conv_gather_tc_supported(p) ? FewTiles::split : FewTiles::gather;
+  }
+  // estimates in ns, fitted to the figures above
+  const double split = igemm_split_estimate(c, p);
+  const double persistent = few ? 1e30 : 2700 + p.Cin * 384 / 95.0;
+  const double best = split >= 0 && split < persistent ? split : persistent;
+  if (!(c.opt_tune & 16) && gemm_fewrows_supported(p)) {
+    // a round: each of a CTA's eight warps takes a row, 512 bytes of it at a time; an SM's CTAs overlap only partly
+    const double rounds = M >= 8 ? (double)((M + 7) / 8) : 0.4 + 0.075 * (double)M, waves = 0.6 * ((p.Cout + 7) / 8) / sms;
+    const double rows = 2000 + (double)p.Cout * p.Cin / 9000 +
+                        rounds * (110 + (p.Cin + 511) / 512 * 512 * 0.58) * (waves > 1 ? waves : 1);
+    if (rows < best) return FewTiles::rows;
+  }
+  return tiles <= sms && split >= 0 && split < persistent ? FewTiles::split : FewTiles::none;
+}
+
 bool launch_conv(Context &c, const ConvProblem &p)
 {
-  if (!c.opt_force_generic && c.opt_split_k == 0 && !(c.opt_tune & 16) && gemm_fewrows_supported(p)) return launch_gemm_fewrows(c, p);
+  switch (few_tiles_form(c, p)) {
+    case FewTiles::rows: return launch_gemm_fewrows(c, p);
+    case FewTiles::gather: return launch_conv_gather_tc(c, p);
+    case FewTiles::split: return launch_igemm_split(c, p);
+    default: break;
+  }
   // The SM-pair kernel: measured equal to the one-CTA kernel for K = 512 (0.054 against 0.053 ms on
   // 14x14x512 -> 512 at batch 1024) and 3-5 % faster for K = 1024 (0.047 against 0.049 ms on 7x7x1024 ->
   // 1024), slower below a few hundred rows per SM pair: taken for K >= 1024 and large M, or on request.

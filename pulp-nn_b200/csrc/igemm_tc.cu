@@ -35,7 +35,7 @@
 //                      eight warps that alternate tiles, 256-column tiles by all sixteen.
 // All 512 columns of tensor memory are used as a ring of 512/BN accumulators, so the MMA issuers run
 // several tiles ahead of the epilogue. Integer accumulation is associative, so splitting K over
-// several CTAs (used when a problem has very few tiles) gives bit-identical sums; partial sums then
+// several CTAs (on request: PULPNN_OPT_SPLIT_K) gives bit-identical sums; partial sums then
 // go to a scratch buffer and a second kernel adds them and requantises. Rows of a short reduction
 // (K <= 64, N <= 64) are folded two or more to a GEMM row against a block-diagonal copy of W (see
 // launch_igemm_tc).
@@ -49,6 +49,7 @@
 
 #include "internal.cuh"
 #include "sm100_primitives.cuh"
+#include "tensor_maps.cuh"
 
 namespace pulpnn {
 
@@ -701,25 +702,6 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const int *partials,
 }
 
 // ---- host side -------------------------------------------------------------------------------
-// [rows][K] byte matrix, K contiguous; box = bkb bytes of K x box_rows rows, bkb-byte swizzle.
-// Elements outside the matrix read as zero.
-bool make_map(CUtensorMap *map, const void *base, int rows, int K, int box_rows, int bkb)
-{
-  EncodeTiledFn enc = encode_tiled_fn();
-  if (!enc) { set_error(PULPNN_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver"); return false; }
-  cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)K};
-  cuuint32_t box[2] = {(cuuint32_t)bkb, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  const CUtensorMapSwizzle sw = bkb == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
-                              : (bkb == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) { set_error(PULPNN_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r); return false; }
-  return true;
-}
-
 // W [N][K] -> block-diagonal [fold*N][fold*K] (block (p, p) = W, zeros elsewhere), 16 bytes per thread
 __global__ void fold_weights_kernel(const int8_t *w, int8_t *wf, int N, int K, int fold)
 {
@@ -733,41 +715,6 @@ __global__ void fold_weights_kernel(const int8_t *w, int8_t *wf, int N, int K, i
     if (pblk == qblk) v = __ldg(reinterpret_cast<const uint4 *>(w + (size_t)n * K + k));
     *reinterpret_cast<uint4 *>(wf + (size_t)row * K * fold + kk) = v;
   }
-}
-
-// [B][H][W][C] image, boxes of box_c bytes x box_w x box_h pixels of one image, every sx-th (sy-th)
-// pixel of the box taken: the pixels one filter tap reads for a patch of outputs
-bool make_map_4d(CUtensorMap *map, const void *base, int C, int Wd, int Hd, int B, int box_c, int box_w, int box_h,
-                 int sx, int sy)
-{
-  EncodeTiledFn enc = encode_tiled_fn();
-  if (!enc) { set_error(PULPNN_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver"); return false; }
-  cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)Wd, (cuuint64_t)Hd, (cuuint64_t)B};
-  cuuint64_t strides[3] = {(cuuint64_t)C, (cuuint64_t)Wd * C, (cuuint64_t)Hd * Wd * C};
-  cuuint32_t box[4] = {(cuuint32_t)box_c, (cuuint32_t)((box_w - 1) * sx + 1), (cuuint32_t)((box_h - 1) * sy + 1), 1};
-  cuuint32_t estr[4] = {1, (cuuint32_t)sx, (cuuint32_t)sy, 1};
-  const CUtensorMapSwizzle sw = box_c == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
-                              : (box_c == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void *>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) { set_error(PULPNN_ERR_CUDA, "cuTensorMapEncodeTiled (4-D) failed with code %d", (int)r); return false; }
-  return true;
-}
-
-// patch width (a power of two, the patch has 128 pixels) that covers the output with the fewest
-// wasted pixels; the wider one on a tie
-int pick_patch_width_log2(int Ho, int Wo, int sx, int sy)
-{
-  int best = -1;
-  long long best_cost = 0;
-  for (int l = 3; l <= 7; l++) {
-    const int tw = 1 << l, th = 128 >> l;
-    if ((tw - 1) * sx + 1 > 256 || (th - 1) * sy + 1 > 256) continue;
-    const long long cost = (long long)((Wo + tw - 1) / tw) * ((Ho + th - 1) / th);
-    if (best < 0 || cost <= best_cost) { best = l; best_cost = cost; }
-  }
-  return best;
 }
 
 // the three tensor maps of a launch (the output map only matters with TMA stores)
@@ -826,12 +773,6 @@ bool launch_final(Context &c, const TcMaps &m, const TcParams &g, int bn, int bk
 
 }  // namespace
 
-// a pointwise convolution or a fully connected layer: A is the plain [M][K] matrix
-static bool igemm_is_plain(const ConvProblem &p)
-{
-  return p.ky == 1 && p.kx == 1 && p.sy == 1 && p.sx == 1 && p.pt == 0 && p.pl == 0 && p.H == p.Ho && p.W == p.Wo;
-}
-
 bool igemm_tc_supported(const Context &c, const ConvProblem &p)
 {
   (void)c;
@@ -843,6 +784,22 @@ bool igemm_tc_supported(const Context &c, const ConvProblem &p)
   if (p.Cin % 32 != 0 || p.ky * p.kx > 121) return false;
   if (p.sx > 16 || p.sy > 16) return false;
   return pick_patch_width_log2(p.Ho, p.Wo, p.sx, p.sy) >= 0 && encode_tiled_fn() != nullptr;
+}
+
+int igemm_tc_tiles(const Context &c, const ConvProblem &p, bool *few)
+{
+  const int sms = c.sm_count > 0 ? c.sm_count : 148;
+  const bool plain = igemm_is_plain(p);
+  const int bkb = plain ? 128 : (p.Cin % 128 == 0 ? 128 : (p.Cin % 64 == 0 ? 64 : 32));
+  const int K = p.ky * p.kx * p.Cin, bn = p.Cout <= 64 ? 64 : (p.Cout <= 128 || K <= 256 ? 128 : 256);
+  long long m = ((long long)p.B * p.Ho * p.Wo + BM - 1) / BM;
+  if (!plain) {
+    const int l = pick_patch_width_log2(p.Ho, p.Wo, p.sx, p.sy);
+    m = (long long)p.B * ((p.Wo + (1 << l) - 1) >> l) * ((p.Ho + (128 >> l) - 1) / (128 >> l));
+  }
+  const long long tiles = m * ((p.Cout + bn - 1) / bn);
+  *few = tiles * 8 <= sms + 8 && (K + bkb - 1) / bkb >= 8;
+  return (int)(tiles < 0x7fffffff ? tiles : 0x7fffffff);
 }
 
 bool launch_igemm_tc(Context &c, const ConvProblem &p)
@@ -919,14 +876,8 @@ bool launch_igemm_tc(Context &c, const ConvProblem &p)
     bn = bn_try;
     g.n_tiles = (g.N + bn - 1) / bn;
     tiles = g.m_tiles * g.n_tiles;
-    // split K only when the tiles alone cannot occupy the GPU and there is enough K to share
-    int slices = 1;
-    if (c.opt_split_k > 0) slices = c.opt_split_k;
-    else if (tiles * 8 <= sms + 8 && g.total_slabs >= 8) {   // measured: from about 32 tiles on the second pass costs more than it saves
-      slices = sms / tiles;
-      if (slices > g.total_slabs / 4) slices = g.total_slabs / 4;
-      if (slices > 16) slices = 16;
-    }
+    // K is split here only on request: problems of few tiles and a long reduction go to igemm_split.cu
+    int slices = c.opt_split_k > 0 ? c.opt_split_k : 1;
     if (slices > g.total_slabs) slices = g.total_slabs;
     if (slices < 1) slices = 1;
     g.slabs_per_slice = (g.total_slabs + slices - 1) / slices;

@@ -245,9 +245,16 @@ bool conv_smallcin_supported(const ConvProblem &p);
 bool launch_conv_smallcin(Context &c, const ConvProblem &p);
 bool igemm_tc_supported(const Context &c, const ConvProblem &p);
 bool launch_igemm_tc(Context &c, const ConvProblem &p);
+// m-tiles x n-tiles that kernel cuts the problem into, and whether these are so few that it leaves the GPU idle over a
+// reduction of eight slabs or more
+int igemm_tc_tiles(const Context &c, const ConvProblem &p, bool *few);
 // the same GEMM computed by pairs of SMs (tcgen05 cta_group::2), for wide layers with a long reduction
 bool igemm_tc2_supported(const Context &c, const ConvProblem &p);
 bool launch_igemm_tc2(Context &c, const ConvProblem &p);
+// the same GEMM for few tiles, the reduction shared by the CTAs of a cluster
+// (estimated ns, or -1 where that kernel does not take the problem)
+double igemm_split_estimate(const Context &c, const ConvProblem &p);
+bool launch_igemm_split(Context &c, const ConvProblem &p);
 // the same contraction for few rows (a fully connected layer at a small batch), on dp4a
 bool gemm_fewrows_supported(const ConvProblem &p);
 bool launch_gemm_fewrows(Context &c, const ConvProblem &p);
@@ -268,6 +275,9 @@ bool launch_dwpw_tcdw(Context &c, const DepthwiseProblem &dw, const ConvProblem 
 bool depthwise_planes_supported(const DepthwiseProblem &p);
 bool launch_depthwise_planes(Context &c, const DepthwiseProblem &p);
 int *ctx_status_word(Context &c);               // allocated on first use; nullptr on failure
+// the same for calls that may come first under a stream capture, where nothing can be allocated: *word stays nullptr
+// then, and a bounded wait that runs out still ends its kernel, unrecorded. false: the allocation failed
+bool ctx_status_word_unless_capturing(Context &c, int **word);
 int static_scratch_status_take(Context &c);     // status of the no-allocation entry point (0: unused or fine)
 bool launch_maxpool(Context &c, const PoolProblem &p, uint8_t *clobber_in);
 bool launch_avgpool(Context &c, const PoolProblem &p);
