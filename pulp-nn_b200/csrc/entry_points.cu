@@ -454,6 +454,23 @@ static FewTiles few_tiles_form(const Context &c, const ConvProblem &p)
   return tiles <= sms && split >= 0 && split < persistent ? FewTiles::split : FewTiles::none;
 }
 
+// Shapes that igemm_tc takes but the gathering kernel runs faster. Output rows that are no whole 16-byte pieces, which
+// igemm_tc stores byte by byte (us, igemm_tc / gather): 56x56x128 -> 100 at batch 64 177 / 26, 28x28x256 -> 250 at batch
+// 32 78 / 12, 18x18x32 -> 77 at batch 59 19.6 / 6.6, 3x3 28x28x64 -> 100 at batch 16 19.7 / 8.6 (equal only for 3x3
+// 14x14x256 -> 77: 20.6 / 21.6). Spatial kernels on channel slabs of 32 bytes, up to 192 output channels: 56x56x96 -> 96
+// at batch 32 43.9 / 27.4, 28x28x160 -> 160 24.9 / 18.8, 56x56x32 -> 64 at batch 64 29.5 / 22.6, 28x28x32 -> 128 11.7 /
+// 11.8; 32 -> 256 13.3 / 16.9, 224 -> 224 18.4 / 19.4. Slabs of 64 bytes, up to 64 channels and enough tiles: 56x56x64
+// -> 64 at batch 64 36.4 / 30.8, at batch 16 13.0 / 12.5; one image 5.3 / 6.7.
+static bool gather_first(const Context &c, const ConvProblem &p)
+{
+  if (c.opt_split_k != 0 || !conv_gather_tc_supported(p)) return false;
+  if (!igemm_tc_whole_rows(c, p)) return true;
+  if (p.ky * p.kx == 1 || p.Cin % 128 == 0) return false;
+  if (p.Cin % 64 != 0) return p.Cout <= 192;
+  bool few;
+  return p.Cout <= 64 && igemm_tc_tiles(c, p, &few) >= 3 * (c.sm_count > 0 ? c.sm_count : 148);
+}
+
 bool launch_conv(Context &c, const ConvProblem &p)
 {
   switch (few_tiles_form(c, p)) {
@@ -468,7 +485,7 @@ bool launch_conv(Context &c, const ConvProblem &p)
   if (!c.opt_force_generic && c.opt_split_k == 0 && igemm_tc2_supported(c, p) &&
       ((c.opt_tune & 8) || (p.Cin >= 1024 && ((long long)p.B * p.Ho * p.Wo / 256) * (p.Cout / 256) >= 4LL * 74)))
     return launch_igemm_tc2(c, p);
-  if (!c.opt_force_generic && igemm_tc_supported(c, p)) return launch_igemm_tc(c, p);
+  if (!c.opt_force_generic && igemm_tc_supported(c, p)) return gather_first(c, p) ? launch_conv_gather_tc(c, p) : launch_igemm_tc(c, p);
   if (!c.opt_force_generic && conv_smallcin_tc_supported(p)) return launch_conv_smallcin_tc(c, p);
   // First layers that the kernel above does not take. conv_smallcin walks the strips of an image in one CTA each:
   // with many small images it beats the gathering kernel (64 images of 28x28x1 -> 16: 4.5 against 6.9 us, of 32x32x3

@@ -786,6 +786,24 @@ bool igemm_tc_supported(const Context &c, const ConvProblem &p)
   return pick_patch_width_log2(p.Ho, p.Wo, p.sx, p.sy) >= 0 && encode_tiled_fn() != nullptr;
 }
 
+// rows of A folded into one row of the GEMM (see launch_igemm_tc): a power of two, 1 for none
+static int fold_of(int M, int N, int K, int sms)
+{
+  if (K > 64 || N > 64 || K % 16 != 0) return 1;
+  int fold = 128 / K < 128 / N ? 128 / K : 128 / N;
+  while (fold > 1 && (fold & (fold - 1))) fold--;
+  while (fold > 1 && (M % fold != 0 || M / (BM * fold) < 2 * sms)) fold /= 2;
+  return fold;
+}
+
+bool igemm_tc_whole_rows(const Context &c, const ConvProblem &p)
+{
+  if (reinterpret_cast<uintptr_t>(p.out) & 15) return false;
+  if (p.epi.mode == EPI_RAW32) return p.Cout % 4 == 0;
+  const int fold = igemm_is_plain(p) ? fold_of(p.B * p.Ho * p.Wo, p.Cout, p.Cin, c.sm_count > 0 ? c.sm_count : 148) : 1;
+  return p.Cout * fold % 16 == 0;
+}
+
 int igemm_tc_tiles(const Context &c, const ConvProblem &p, bool *few)
 {
   const int sms = c.sm_count > 0 ? c.sm_count : 148;
@@ -833,11 +851,7 @@ bool launch_igemm_tc(Context &c, const ConvProblem &p)
     // Measured on 112x112x32 -> 64 at batch 1024: 0.284 ms unfolded, 0.256 ms with two pixels per
     // row (one 128-column tile, TMA stores), 0.261 ms with four; 64 -> 128 channels loses 5 % when
     // folded, so only outputs of at most 64 channels are, up to one 128-column tile.
-    if (g.K <= 64 && g.N <= 64 && g.K % 16 == 0 && c.opt_split_k == 0) {
-      fold = 128 / g.K < 128 / g.N ? 128 / g.K : 128 / g.N;
-      while (fold > 1 && (fold & (fold - 1))) fold--;                    // a power of two
-      while (fold > 1 && (g.M % fold != 0 || g.M / (BM * fold) < 2 * sms)) fold /= 2;
-    }
+    if (c.opt_split_k == 0) fold = fold_of(g.M, g.N, g.K, sms);
     if (fold > 1) {
       const size_t wbytes = (size_t)g.N * fold * g.K * fold;
       int slot = 0;

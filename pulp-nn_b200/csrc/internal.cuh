@@ -245,6 +245,8 @@ bool conv_smallcin_supported(const ConvProblem &p);
 bool launch_conv_smallcin(Context &c, const ConvProblem &p);
 bool igemm_tc_supported(const Context &c, const ConvProblem &p);
 bool launch_igemm_tc(Context &c, const ConvProblem &p);
+// whether its output rows are whole 16-byte pieces; otherwise it stores byte by byte
+bool igemm_tc_whole_rows(const Context &c, const ConvProblem &p);
 // m-tiles x n-tiles that kernel cuts the problem into, and whether these are so few that it leaves the GPU idle over a
 // reduction of eight slabs or more
 int igemm_tc_tiles(const Context &c, const ConvProblem &p, bool *few);
