@@ -296,6 +296,8 @@ __global__ void __launch_bounds__(GT, 2) conv_gather_tc_kernel(const __grid_cons
             if (mb + rr < g.M && col < ncols) o[(size_t)(mb + rr) * p.Cout] = tile[rr * 33 + lane];
         } else {
           unsigned w[8];
+          const bool fits = MODE == EPI_BN64 &&
+              __all_sync(0xffffffffu, c0 + lane >= ncols || bn_fits_32(par_k[c0 + lane], par_l[c0 + lane], acc_bound(g.K), e.shift));
 #pragma unroll
           for (int j = 0; j < 32; j += 4) {
             int t[4];
@@ -308,10 +310,7 @@ __global__ void __launch_bounds__(GT, 2) conv_gather_tc_kernel(const __grid_cons
               t[2] = (int)((unsigned)kk.z * v[j + 2] + (unsigned)ll.z) >> e.shift;
               t[3] = (int)((unsigned)kk.w * v[j + 3] + (unsigned)ll.w) >> e.shift;
             } else if (MODE == EPI_BN64) {
-#pragma unroll
-              for (int u = 0; u < 4; u++)
-                t[u] = (int)((long long)((unsigned long long)par_k[c0 + j + u] * (unsigned long long)(long long)(int)v[j + u] +
-                                         (unsigned long long)par_l[c0 + j + u]) >> e.shift);
+              requant4_bn64(par_k + c0 + j, par_l + c0 + j, v[j], v[j + 1], v[j + 2], v[j + 3], e.shift, fits, t);
             } else {
               const int4 bb = *reinterpret_cast<const int4 *>(reinterpret_cast<const int *>(par_l) + c0 + j);
               const int a4[4] = {(int)v[j] + bb.x, (int)v[j + 1] + bb.y, (int)v[j + 2] + bb.z, (int)v[j + 3] + bb.w};

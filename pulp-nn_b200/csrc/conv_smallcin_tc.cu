@@ -257,13 +257,23 @@ conv_smallcin_tc_kernel(const __grid_constant__ CUtensorMap map_in, const SmallT
     const int ox = quad * 32 + lane;
     // 32 filters with 32-bit batch normalisation: k and lambda live in registers for the CTA's
     // lifetime, so a tile costs one multiply-add and one shift per output and no parameter loads
-    constexpr bool REG_PARAMS = MODE == EPI_BN32 && BN == 32;
+    // (64-bit parameters too, where 32-bit arithmetic gives the same: bn_fits_32)
+    constexpr bool REG_PARAMS = (MODE == EPI_BN32 || MODE == EPI_BN64) && BN == 32;
+    bool fits = MODE == EPI_BN32;
+    if (MODE == EPI_BN64) {
+      bool mine = true;
+      for (int n = lane; n < BN; n += 32)
+        mine = mine && bn_fits_32(reinterpret_cast<const long long *>(params)[n], reinterpret_cast<const long long *>(params)[BN + n],
+                                  27 * ACC_PER_TERM, e.shift);
+      fits = __all_sync(0xffffffffu, mine);
+    }
     int kr[32], lr[32];
     if (REG_PARAMS) {
 #pragma unroll
       for (int j = 0; j < 32; j++) {
-        kr[j] = reinterpret_cast<const int *>(params)[j];
-        lr[j] = reinterpret_cast<const int *>(params)[BN + j];
+        // a 64-bit value's low word
+        kr[j] = reinterpret_cast<const int *>(params)[MODE == EPI_BN64 ? 2 * j : j];
+        lr[j] = reinterpret_cast<const int *>(params)[MODE == EPI_BN64 ? 2 * (BN + j) : BN + j];
       }
     }
     int i = 0;
@@ -290,7 +300,7 @@ conv_smallcin_tc_kernel(const __grid_constant__ CUtensorMap map_in, const SmallT
 #pragma unroll
           for (int j = 0; j < 32; j += 4) {
             int q[4];
-            if (REG_PARAMS) {
+            if (REG_PARAMS && fits) {
 #pragma unroll
               for (int t = 0; t < 4; t++) q[t] = (int)((unsigned)kr[j + t] * v[j + t] + (unsigned)lr[j + t]) >> e.shift;
             } else if (MODE == EPI_BN32) {
@@ -300,15 +310,14 @@ conv_smallcin_tc_kernel(const __grid_constant__ CUtensorMap map_in, const SmallT
               q[1] = (int)((unsigned)kk.y * v[j + 1] + (unsigned)ll.y) >> e.shift;
               q[2] = (int)((unsigned)kk.z * v[j + 2] + (unsigned)ll.z) >> e.shift;
               q[3] = (int)((unsigned)kk.w * v[j + 3] + (unsigned)ll.w) >> e.shift;
+            } else if (MODE == EPI_BN64) {
+              requant4_bn64(reinterpret_cast<const long long *>(params) + c0 + j, reinterpret_cast<const long long *>(params) + BN + c0 + j,
+                            v[j], v[j + 1], v[j + 2], v[j + 3], e.shift, fits, q);
             } else {
 #pragma unroll
               for (int t = 0; t < 4; t++) {
                 const int acc = (int)v[j + t];
-                if (MODE == EPI_BN64) {
-                  const long long k = reinterpret_cast<const long long *>(params)[c0 + j + t];
-                  const long long l = reinterpret_cast<const long long *>(params)[BN + c0 + j + t];
-                  q[t] = (int)((long long)((unsigned long long)k * (unsigned long long)(long long)acc + (unsigned long long)l) >> e.shift);
-                } else if (MODE == EPI_MULT) {
+                if (MODE == EPI_MULT) {
                   q[t] = (int)(short)((int)((unsigned)e.out_mult * (unsigned)(acc + reinterpret_cast<const int *>(params)[c0 + j + t])) >> e.shift);
                 } else {
                   q[t] = (acc + reinterpret_cast<const int *>(params)[c0 + j + t]) >> e.shift;

@@ -70,7 +70,8 @@ struct HwcTmaParams {
 };
 
 // requantise a completed 4 columns x 4 channels block and put the four pixel words in the tile
-template <int MODE, bool K32, int CI>
+// WIDE: 0 64-bit arithmetic, 1 every k fits in 32 bits, 2 32-bit arithmetic gives the same (bn_fits_32)
+template <int MODE, int WIDE, int CI>
 __device__ __forceinline__ void finalize_k(const int (&acc)[4][4], const QuantT<MODE> &q, const Epilogue &e, uint32_t oaddr)
 {
 #pragma unroll
@@ -78,9 +79,9 @@ __device__ __forceinline__ void finalize_k(const int (&acc)[4][4], const QuantT<
     int v[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      if (MODE == EPI_BN32)
+      if (MODE == EPI_BN32 || (MODE == EPI_BN64 && WIDE == 2))
         v[j] = (int)((unsigned)q.k[j] * (unsigned)acc[i][j] + (unsigned)q.l[j]) >> e.shift;
-      else if (MODE == EPI_BN64 && K32)      // every k fits in 32 bits: one wide multiply-add
+      else if (MODE == EPI_BN64 && WIDE == 1)      // every k fits in 32 bits: one wide multiply-add
         v[j] = (int)(mad_wide_s32((int)q.k[j], acc[i][j], (long long)q.l[j]) >> e.shift);
       else if (MODE == EPI_BN64)
         v[j] = (int)((long long)((unsigned long long)q.k[j] * (unsigned long long)(long long)acc[i][j] +
@@ -95,10 +96,11 @@ __device__ __forceinline__ void finalize_k(const int (&acc)[4][4], const QuantT<
 }
 template <int MODE, int CI>
 __device__ __forceinline__ void finalize_row(const int (&acc)[4][4], const QuantT<MODE> &q, const Epilogue &e,
-                                             bool k32, uint32_t oaddr)
+                                             int wide, uint32_t oaddr)
 {
-  if (MODE == EPI_BN64 && k32) finalize_k<MODE, true, CI>(acc, q, e, oaddr);
-  else finalize_k<MODE, false, CI>(acc, q, e, oaddr);
+  if (MODE == EPI_BN64 && wide == 2) finalize_k<MODE, 2, CI>(acc, q, e, oaddr);
+  else if (MODE == EPI_BN64 && wide == 1) finalize_k<MODE, 1, CI>(acc, q, e, oaddr);
+  else finalize_k<MODE, 0, CI>(acc, q, e, oaddr);
 }
 
 template <int MODE, int S, int NGX, int CI>
@@ -170,7 +172,7 @@ depthwise_hwc3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const __
   }
   QuantT<MODE> q;
   int init[4];
-  bool k32 = true;
+  int wide = 2;
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     q.bias[j] = e.bias ? (int)__ldg(reinterpret_cast<const int8_t *>(e.bias) + c + j) : 0;
@@ -185,7 +187,7 @@ depthwise_hwc3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const __
       q.k[j] = k;
       q.l[j] = (long long)((unsigned long long)k * (unsigned long long)(long long)q.bias[j] +
                            (unsigned long long)__ldg(reinterpret_cast<const long long *>(e.lambda) + c + j));
-      k32 = k32 && (k == (long long)(int)k);
+      wide = min(wide, bn_fits_32(k, (long long)q.l[j], 9 * ACC_PER_TERM, e.shift) ? 2 : (k == (long long)(int)k ? 1 : 0));
     }
   }
   // The filter taps and requantisation parameters above are constants, fetched while the previous
@@ -252,16 +254,16 @@ depthwise_hwc3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const __
           windows1(cur, rot, w);
           if (rows_here > 1) load_row1<CI>(ia, ra, G::IN_PITCH, cur);
           mac1<true, true>(w, wa, wb, init, acc[0], acc[A1], acc[A2]);
-          finalize_row<MODE, CI>(acc[0], q, e, k32, oa);
+          finalize_row<MODE, CI>(acc[0], q, e, wide, oa);
           if (rows_here > 1) {            // the strip's last group may end before its third row
             windows1(cur, rot, w);
             if (rows_here > 2) load_row1<CI>(ia, ra, 2 * G::IN_PITCH, cur);
             mac1<true, true>(w, wa, wb, init, acc[A1], acc[A2], acc[0]);
-            finalize_row<MODE, CI>(acc[A1], q, e, k32, oa + G::OUT_PITCH);
+            finalize_row<MODE, CI>(acc[A1], q, e, wide, oa + G::OUT_PITCH);
             if (rows_here > 2) {
               windows1(cur, rot, w);
               mac1<true, true>(w, wa, wb, init, acc[A2], acc[0], acc[A1]);
-              finalize_row<MODE, CI>(acc[A2], q, e, k32, oa + 2 * G::OUT_PITCH);
+              finalize_row<MODE, CI>(acc[A2], q, e, wide, oa + 2 * G::OUT_PITCH);
             }
           }
         } else {
@@ -273,7 +275,7 @@ depthwise_hwc3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const __
           windows2(cur, rot, w);
           if (rows_here > 1) load_row2<CI>(ia, ra, 2 * G::IN_PITCH, cur);
           mac2<false>(w, wa[2], wb[2], init, acc[0]);
-          finalize_row<MODE, CI>(acc[0], q, e, k32, oa);
+          finalize_row<MODE, CI>(acc[0], q, e, wide, oa);
           if (rows_here > 1) {
             mac2<true>(w, wa[0], wb[0], init, acc[0]);
             windows2(cur, rot, w);
@@ -281,7 +283,7 @@ depthwise_hwc3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const __
             mac2<false>(w, wa[1], wb[1], init, acc[0]);
             windows2(cur, rot, w);
             mac2<false>(w, wa[2], wb[2], init, acc[0]);
-            finalize_row<MODE, CI>(acc[0], q, e, k32, oa + G::OUT_PITCH);
+            finalize_row<MODE, CI>(acc[0], q, e, wide, oa + G::OUT_PITCH);
             mac2<true>(w, wa[0], wb[0], init, acc[0]);
           }
         }
@@ -437,7 +439,7 @@ depthwise_chw3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const Ch
   }
   QuantT<MODE> q;
   int init[4];
-  bool k32 = true;
+  int wide = 2;
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     q.bias[j] = e.bias ? (int)__ldg(reinterpret_cast<const int8_t *>(e.bias) + c + j) : 0;
@@ -452,7 +454,7 @@ depthwise_chw3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const Ch
       q.k[j] = k;
       q.l[j] = (long long)((unsigned long long)k * (unsigned long long)(long long)q.bias[j] +
                            (unsigned long long)__ldg(reinterpret_cast<const long long *>(e.lambda) + c + j));
-      k32 = k32 && (k == (long long)(int)k);
+      wide = min(wide, bn_fits_32(k, (long long)q.l[j], 9 * ACC_PER_TERM, e.shift) ? 2 : (k == (long long)(int)k ? 1 : 0));
     }
   }
   __syncthreads();                                   // the barriers are initialised
@@ -534,15 +536,15 @@ depthwise_chw3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const Ch
         Win1 w;
         load_win_chw(ia, 0, lmask, rmask, w);
         mac1<true, true>(w, wa, wb, init, acc[0], acc[A1], acc[A2]);
-        finalize_row<MODE, G::PP>(acc[0], q, e, k32, oa);
+        finalize_row<MODE, G::PP>(acc[0], q, e, wide, oa);
         if (rows_here > 1) {
           load_win_chw(ia, W, lmask, rmask, w);
           mac1<true, true>(w, wa, wb, init, acc[A1], acc[A2], acc[0]);
-          finalize_row<MODE, G::PP>(acc[A1], q, e, k32, oa + G::OUT_PITCH);
+          finalize_row<MODE, G::PP>(acc[A1], q, e, wide, oa + G::OUT_PITCH);
           if (rows_here > 2) {
             load_win_chw(ia, 2 * W, lmask, rmask, w);
             mac1<true, true>(w, wa, wb, init, acc[A2], acc[0], acc[A1]);
-            finalize_row<MODE, G::PP>(acc[A2], q, e, k32, oa + 2 * G::OUT_PITCH);
+            finalize_row<MODE, G::PP>(acc[A2], q, e, wide, oa + 2 * G::OUT_PITCH);
           }
         }
       } else {
@@ -552,13 +554,13 @@ depthwise_chw3x3_tma_kernel(const __grid_constant__ CUtensorMap map_in, const Ch
         mac2<false>(w, wa[1], wb[1], init, acc[0]);
         if (rows_here > 1) load_win_chw(ia, 2 * W, lmask, rmask, w);
         mac2<false>(v, wa[2], wb[2], init, acc[0]);
-        finalize_row<MODE, G::PP>(acc[0], q, e, k32, oa);
+        finalize_row<MODE, G::PP>(acc[0], q, e, wide, oa);
         if (rows_here > 1) {
           mac2<true>(v, wa[0], wb[0], init, acc[0]);
           load_win_chw(ia, 3 * W, lmask, rmask, v);
           mac2<false>(w, wa[1], wb[1], init, acc[0]);
           mac2<false>(v, wa[2], wb[2], init, acc[0]);
-          finalize_row<MODE, G::PP>(acc[0], q, e, k32, oa + G::OUT_PITCH);
+          finalize_row<MODE, G::PP>(acc[0], q, e, wide, oa + G::OUT_PITCH);
           mac2<true>(v, wa[0], wb[0], init, acc[0]);
         }
       }

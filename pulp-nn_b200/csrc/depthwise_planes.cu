@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
     ll = __ldg(reinterpret_cast<const long long *>(e.lambda) + c);
   }
   const int bias = e.bias ? (int)__ldg(reinterpret_cast<const int8_t *>(e.bias) + c) : 0;
+  const bool fits = MODE == EPI_BN64 && __all_sync(0xffffffffu, bn_fits_32(kk, ll, K * K * ACC_PER_TERM + 128, e.shift));
   __syncthreads();
 
   // ---- compute: a unit is four columns x R rows of the warp's channels ------------------------------
@@ -210,7 +211,8 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
         if (oy + r >= p.Ho) break;
 #pragma unroll
         for (int i = 0; i < 4; i++)
-          if (ox + i < p.Wo) o[((size_t)r * p.Wo + i) * p.C] = (uint8_t)requant_kl<MODE>(acc[r][i], kk, ll, e.out_mult, e.shift);
+          if (ox + i < p.Wo) o[((size_t)r * p.Wo + i) * p.C] = (uint8_t)(fits ? requant_kl<EPI_BN32>(acc[r][i], kk, ll, e.out_mult, e.shift)
+                                                            : requant_kl<MODE>(acc[r][i], kk, ll, e.out_mult, e.shift));
       }
     }
   }

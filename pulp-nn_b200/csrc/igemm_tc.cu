@@ -425,6 +425,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     long long *p_k64 = reinterpret_cast<long long *>(params);      // EPI_BN64
     long long *p_l64 = p_k64 + HALF_COLS;
     int staged_nt = -1;
+    bool fits = false;                                             // EPI_BN64: 32-bit arithmetic gives the same (internal.cuh)
     // TMA_OUT: the group's staging tile, and the one thread of the group that issues its stores
     uint8_t *out_tile = smem + L::OUT_OFFSET + grp * L::OUT_TILE_BYTES;
     const bool elected = ((warp - FIRST_EPI) % (4 * NSPLIT)) == 0 && lane == 0;
@@ -442,6 +443,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         // lambda: k*(acc+b)+lambda == k*acc + (k*b+lambda) in wrap-around arithmetic.
         // Local slot i holds column (i/32)*32*NSPLIT + half*32 + i%32 of the tile.
         __syncwarp();
+        bool mine = true;
         for (int i = lane; i < HALF_COLS; i += 32) {
           const int col = n0 + (i >> 5) * (32 * NSPLIT) + half * 32 + (i & 31);
           const bool v = col < g.N;
@@ -457,12 +459,24 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             const long long l = v ? __ldg(reinterpret_cast<const long long *>(e.lambda) + n) : 0;
             const long long b = (v && e.bias) ? (long long)__ldg(reinterpret_cast<const int8_t *>(e.bias) + n) : 0;
             p_k64[i] = k;
-            p_l64[i] = (long long)((unsigned long long)k * (unsigned long long)b + (unsigned long long)l);
+            const long long lb = (long long)((unsigned long long)k * (unsigned long long)b + (unsigned long long)l);
+            p_l64[i] = lb;
+            mine = mine && bn_fits_32(k, lb, acc_bound(g.K), e.shift);
           } else if (MODE == EPI_RAW32) {
             p_bias[i] = (v && e.bias) ? __ldg(reinterpret_cast<const int *>(e.bias) + n) : 0;
           } else {
             p_bias[i] = (v && e.bias) ? (int)__ldg(reinterpret_cast<const int8_t *>(e.bias) + n) : 0;
           }
+        }
+        fits = MODE == EPI_BN64 && __all_sync(0xffffffffu, mine);
+        if (MODE == EPI_BN64 && fits) {
+          // stored again as 32-bit values, the way the 32-bit epilogue reads them
+          static_assert(HALF_COLS <= 64, "two columns per lane");
+          const int i1 = lane + 32 < HALF_COLS ? lane + 32 : lane;
+          const int ka = (int)p_k64[lane], kb = (int)p_k64[i1], la = (int)p_l64[lane], lb = (int)p_l64[i1];
+          __syncwarp();
+          p_k32[lane] = ka; p_l32[lane] = la;
+          if (i1 != lane) { p_k32[i1] = kb; p_l32[i1] = lb; }
         }
         __syncwarp();
         staged_nt = nt;
@@ -502,21 +516,20 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
               for (int j = 0; j < 32; j += 4) {
                 int q[4];
-                if (MODE == EPI_BN32) {
+                if (MODE == EPI_BN32 || (MODE == EPI_BN64 && fits)) {
                   const int4 kk = *reinterpret_cast<const int4 *>(p_k32 + lc + j);
                   const int4 ll = *reinterpret_cast<const int4 *>(p_l32 + lc + j);
                   q[0] = (int)((unsigned)kk.x * v[j + 0] + (unsigned)ll.x) >> e.shift;
                   q[1] = (int)((unsigned)kk.y * v[j + 1] + (unsigned)ll.y) >> e.shift;
                   q[2] = (int)((unsigned)kk.z * v[j + 2] + (unsigned)ll.z) >> e.shift;
                   q[3] = (int)((unsigned)kk.w * v[j + 3] + (unsigned)ll.w) >> e.shift;
+                } else if (MODE == EPI_BN64) {
+                  requant4_bn64(p_k64 + lc + j, p_l64 + lc + j, v[j], v[j + 1], v[j + 2], v[j + 3], e.shift, false, q);
                 } else {
 #pragma unroll
                   for (int t = 0; t < 4; t++) {
                     const int a = (int)v[j + t];
-                    if (MODE == EPI_BN64)
-                      q[t] = (int)((long long)((unsigned long long)p_k64[lc + j + t] * (unsigned long long)(long long)a +
-                                               (unsigned long long)p_l64[lc + j + t]) >> e.shift);
-                    else if (MODE == EPI_MULT)
+                    if (MODE == EPI_MULT)
                       q[t] = (int)(short)((int)((unsigned)e.out_mult * (unsigned)(a + p_bias[lc + j + t])) >> e.shift);
                     else
                       q[t] = (a + p_bias[lc + j + t]) >> e.shift;
@@ -619,21 +632,20 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
             int q[4];
-            if (MODE == EPI_BN32) {
+            if (MODE == EPI_BN32 || (MODE == EPI_BN64 && fits)) {
               const int4 kk = *reinterpret_cast<const int4 *>(p_k32 + lc + i);
               const int4 ll = *reinterpret_cast<const int4 *>(p_l32 + lc + i);
               q[0] = (int)((unsigned)kk.x * v[i + 0] + (unsigned)ll.x) >> e.shift;
               q[1] = (int)((unsigned)kk.y * v[i + 1] + (unsigned)ll.y) >> e.shift;
               q[2] = (int)((unsigned)kk.z * v[i + 2] + (unsigned)ll.z) >> e.shift;
               q[3] = (int)((unsigned)kk.w * v[i + 3] + (unsigned)ll.w) >> e.shift;
+            } else if (MODE == EPI_BN64) {
+              requant4_bn64(p_k64 + lc + i, p_l64 + lc + i, v[i], v[i + 1], v[i + 2], v[i + 3], e.shift, false, q);
             } else {
 #pragma unroll
               for (int j = 0; j < 4; j++) {
                 const int a = (int)v[i + j];
-                if (MODE == EPI_BN64)
-                  q[j] = (int)((long long)((unsigned long long)p_k64[lc + i + j] * (unsigned long long)(long long)a +
-                                           (unsigned long long)p_l64[lc + i + j]) >> e.shift);
-                else if (MODE == EPI_MULT)
+                if (MODE == EPI_MULT)
                   q[j] = (int)(short)((int)((unsigned)e.out_mult * (unsigned)(a + p_bias[lc + i + j])) >> e.shift);
                 else
                   q[j] = (a + p_bias[lc + i + j]) >> e.shift;

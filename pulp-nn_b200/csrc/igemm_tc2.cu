@@ -169,6 +169,7 @@ igemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   if (warp == 1) tmem_alloc_pair(tmem_slot, 512);
   // per-channel parameters of the cluster's columns -> shared memory, once; the bias is folded into
   // lambda: k*(acc+b)+lambda == k*acc + (k*b+lambda) in wrap-around arithmetic
+  bool mine = true;                 // EPI_BN64: 32-bit arithmetic gives the same for this thread's channels
   for (int i = threadIdx.x; i < g.nt * BN; i += THREADS2) {
     const int n = n_base + i;
     const int bias8 = e.bias ? (int)__ldg(reinterpret_cast<const int8_t *>(e.bias) + n) : 0;
@@ -180,15 +181,16 @@ igemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     } else if (MODE == EPI_BN64) {
       const long long k = __ldg(reinterpret_cast<const long long *>(e.k) + n);
       reinterpret_cast<long long *>(params)[i] = k;
-      reinterpret_cast<long long *>(params)[g.nt * BN + i] =
-          (long long)((unsigned long long)k * (unsigned long long)(long long)bias8 +
-                      (unsigned long long)__ldg(reinterpret_cast<const long long *>(e.lambda) + n));
+      const long long l = (long long)((unsigned long long)k * (unsigned long long)(long long)bias8 +
+                                      (unsigned long long)__ldg(reinterpret_cast<const long long *>(e.lambda) + n));
+      reinterpret_cast<long long *>(params)[g.nt * BN + i] = l;
+      mine = mine && bn_fits_32(k, l, acc_bound(g.K), e.shift);
     } else {
       reinterpret_cast<int *>(params)[i] = bias8;
     }
   }
   tc_fence_before();
-  __syncthreads();
+  const bool fits = __syncthreads_and(mine);
   // both CTAs' barriers are initialised before either signals the other's
   cluster_sync_all();
   tc_fence_after();
@@ -315,14 +317,13 @@ igemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 q[1] = (int)((unsigned)kk.y * v[j + 1] + (unsigned)ll.y) >> e.shift;
                 q[2] = (int)((unsigned)kk.z * v[j + 2] + (unsigned)ll.z) >> e.shift;
                 q[3] = (int)((unsigned)kk.w * v[j + 3] + (unsigned)ll.w) >> e.shift;
+              } else if (MODE == EPI_BN64) {
+                requant4_bn64(p_k64 + pc + j, p_l64 + pc + j, v[j], v[j + 1], v[j + 2], v[j + 3], e.shift, fits, q);
               } else {
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                   const int a = (int)v[j + u];
-                  if (MODE == EPI_BN64)
-                    q[u] = (int)((long long)((unsigned long long)p_k64[pc + j + u] * (unsigned long long)(long long)a +
-                                             (unsigned long long)p_l64[pc + j + u]) >> e.shift);
-                  else if (MODE == EPI_MULT)
+                  if (MODE == EPI_MULT)
                     q[u] = (int)(short)((int)((unsigned)e.out_mult * (unsigned)(a + p_bias[pc + j + u])) >> e.shift);
                   else
                     q[u] = (a + p_bias[pc + j + u]) >> e.shift;

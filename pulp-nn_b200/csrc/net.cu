@@ -16,6 +16,7 @@ struct Layer {
   pulpnn_layer_desc_t d;
   const int8_t *w = nullptr;
   const void *bias = nullptr, *k = nullptr, *lambda = nullptr;
+  const void *k32 = nullptr, *lambda32 = nullptr;   // 64-bit parameters whose 32-bit copies give the same results
   size_t in_bytes = 0, out_bytes = 0;      // per image
   int mode = EPI_NONE;
   FoldedWeights folded;                    // device copies owned by the network
@@ -67,19 +68,63 @@ const void *upload(pulpnn_net *net, const void *src, size_t bytes)
   return dev;
 }
 
-Epilogue layer_epilogue(const Layer &L)
+// 32-bit copies of a layer's 64-bit batch-norm parameters, where the 32-bit arithmetic gives the same results: for no
+// sum the layer's weights and bias can produce does k*acc + lambda leave the int32 range, and the shift fits. The
+// kernels of the 32-bit tree then serve the layer (their epilogues take about a third of the instructions).
+bool narrow_parameters(pulpnn_net *net, Layer &L, const pulpnn_layer_desc_t &d, size_t wbytes)
+try {
+  const int n = d.ch_out;
+  if (d.out_shift > 31) return true;
+  // the caller's arrays where they are in host memory, copies of the device ones otherwise
+  std::vector<std::vector<char>> copies;
+  auto host = [&](const void *src, size_t bytes) -> const void * {
+    if (!src || !is_device_ptr(src)) return src;
+    copies.emplace_back(bytes);
+    return cuda_ok(cudaMemcpy(copies.back().data(), src, bytes, cudaMemcpyDeviceToHost), "parameter check") ? copies.back().data() : nullptr;
+  };
+  const long long *k = static_cast<const long long *>(host(d.k, 8 * (size_t)n));
+  const long long *l = static_cast<const long long *>(host(d.lambda, 8 * (size_t)n));
+  const int8_t *bias = static_cast<const int8_t *>(host(d.bias, n)), *w = nullptr;
+  if (!k || !l || (d.bias && !bias)) return false;
+  const size_t terms = wbytes / n;
+  std::vector<int> k32(n), l32(n);
+  for (int c = 0; c < n; c++) {
+    const long long lim = 0x7fffffffLL;
+    if (k[c] > lim || k[c] < -lim || l[c] > lim || l[c] < -lim) return true;
+    const long long ak = k[c] < 0 ? -k[c] : k[c], al = l[c] < 0 ? -l[c] : l[c];
+    // first with the largest weights there can be, then with the channel's own
+    long long sum = (long long)terms * 128 * 255 + 128;
+    if (terms > 65535) return true;
+    if (ak * sum + al > lim) {
+      if (!w) w = static_cast<const int8_t *>(host(d.weights, wbytes));
+      if (!w) return false;
+      sum = bias ? (bias[c] < 0 ? -bias[c] : bias[c]) : 0;
+      for (size_t i = 0; i < terms; i++) sum += 255LL * (w[c * terms + i] < 0 ? -w[c * terms + i] : w[c * terms + i]);
+      if (ak * sum + al > lim) return true;
+    }
+    k32[c] = (int)k[c]; l32[c] = (int)l[c];
+  }
+  L.k32 = upload(net, k32.data(), 4 * (size_t)n);
+  L.lambda32 = upload(net, l32.data(), 4 * (size_t)n);
+  return L.k32 && L.lambda32;
+} catch (const std::bad_alloc &) {
+  return true;                        // no memory to look: the 64-bit parameters serve
+}
+
+Epilogue layer_epilogue(const Layer &L, bool narrow = true)
 {
   Epilogue e;
   e.k = L.k; e.lambda = L.lambda; e.bias = L.bias; e.mode = L.mode;
+  if (narrow && L.k32) { e.k = L.k32; e.lambda = L.lambda32; e.mode = EPI_BN32; }
   e.out_mult = (int)(int16_t)(uint16_t)L.d.out_mult; e.shift = L.d.out_shift;
   return e;
 }
 
-ConvProblem conv_problem(Layer &L, const uint8_t *in, void *out, int n)
+ConvProblem conv_problem(Layer &L, const uint8_t *in, void *out, int n, bool narrow = true)
 {
   const pulpnn_layer_desc_t &d = L.d;
   ConvProblem p;
-  p.in = in; p.w = L.w; p.out = out; p.epi = layer_epilogue(L); p.folded = &L.folded;
+  p.in = in; p.w = L.w; p.out = out; p.epi = layer_epilogue(L, narrow); p.folded = &L.folded;
   p.B = n; p.H = d.dim_in_y; p.W = d.dim_in_x; p.Cin = d.ch_in; p.Ho = d.dim_out_y; p.Wo = d.dim_out_x;
   p.Cout = d.ch_out;
   if (d.type == PULPNN_LAYER_CONV) {
@@ -91,11 +136,11 @@ ConvProblem conv_problem(Layer &L, const uint8_t *in, void *out, int n)
   return p;
 }
 
-DepthwiseProblem depthwise_problem(const Layer &L, const uint8_t *in, void *out, int n)
+DepthwiseProblem depthwise_problem(const Layer &L, const uint8_t *in, void *out, int n, bool narrow = true)
 {
   const pulpnn_layer_desc_t &d = L.d;
   DepthwiseProblem p;
-  p.in = in; p.w = L.w; p.out = static_cast<uint8_t *>(out); p.epi = layer_epilogue(L);
+  p.in = in; p.w = L.w; p.out = static_cast<uint8_t *>(out); p.epi = layer_epilogue(L, narrow);
   p.B = n; p.H = d.dim_in_y; p.W = d.dim_in_x; p.C = d.ch_in; p.Ho = d.dim_out_y; p.Wo = d.dim_out_x;
   p.ky = d.dim_kernel_y; p.kx = d.dim_kernel_x; p.pt = d.padding_y_top; p.pl = d.padding_x_left;
   p.sy = d.stride_y; p.sx = d.stride_x; p.in_is_hwc = true;
@@ -128,6 +173,9 @@ bool run_layer(Context &c, const pulpnn_net *net, Layer &L, const uint8_t *in, v
   }
 }
 
+// a fused kernel has one requantisation mode: a pair takes its 32-bit parameters only if both layers have them
+bool pair_is_narrow(const Layer &A, const Layer &B) { return A.k32 && B.k32; }
+
 // Layers l (depthwise) and l+1 (pointwise) as one kernel, the depthwise output never leaving the
 // SM? Only where a fused kernel exists for the pair's shape and both layers requantise the same way.
 bool pair_is_fusable(Context &c, pulpnn_net *net, int l, int n_layers, const uint8_t *in, void *out, int n)
@@ -135,7 +183,8 @@ bool pair_is_fusable(Context &c, pulpnn_net *net, int l, int n_layers, const uin
   if (!c.opt_fuse_dwpw || l + 1 >= n_layers) return false;
   Layer &A = net->layers[l], &B = net->layers[l + 1];
   if (A.d.type != PULPNN_LAYER_DEPTHWISE || B.d.type != PULPNN_LAYER_POINTWISE) return false;
-  return dwpw_fused_supported(depthwise_problem(A, in, nullptr, n), conv_problem(B, nullptr, out, n));
+  const bool narrow = pair_is_narrow(A, B);
+  return dwpw_fused_supported(depthwise_problem(A, in, nullptr, n, narrow), conv_problem(B, nullptr, out, n, narrow));
 }
 
 // pushes images [0, n) that already sit in device memory through layers [0, n_layers)
@@ -168,8 +217,9 @@ bool run_device(Context &c, pulpnn_net *net, const uint8_t *din, uint8_t *dout, 
       if (!mark()) return false;
       if (pair_is_fusable(c, net, l, n_layers, cur, dest(l + 1), nb)) {
         void *dst = dest(l + 1);
-        if (!launch_dwpw_fused(c, depthwise_problem(net->layers[l], cur, nullptr, nb),
-                               conv_problem(net->layers[l + 1], nullptr, dst, nb)))
+        const bool narrow = pair_is_narrow(net->layers[l], net->layers[l + 1]);
+        if (!launch_dwpw_fused(c, depthwise_problem(net->layers[l], cur, nullptr, nb, narrow),
+                               conv_problem(net->layers[l + 1], nullptr, dst, nb, narrow)))
           return false;
         cur = static_cast<const uint8_t *>(dst);
         cur_buf = other;
@@ -377,6 +427,7 @@ int pulpnn_net_add_layer(pulpnn_net_t *net, const pulpnn_layer_desc_t *desc)
       L.k = upload(net, d.k, bn_sz * d.ch_out);
       L.lambda = upload(net, d.lambda, bn_sz * d.ch_out);
       if (!L.k || !L.lambda) return c.err;
+      if (L.mode == EPI_BN64 && !narrow_parameters(net, L, d, wbytes)) return c.err;
     }
   }
   L.d.weights = nullptr; L.d.bias = nullptr; L.d.k = L.d.lambda = nullptr;
