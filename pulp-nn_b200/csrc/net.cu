@@ -249,13 +249,21 @@ bool run_device(Context &c, pulpnn_net *net, const uint8_t *din, uint8_t *dout, 
 // Host input: copied in a few slices on a second stream, each slice going through the whole stack as
 // soon as it has landed, so that the copy of slice i+1 overlaps the compute of slice i. With a
 // micro-batch set, a slice is a whole number of micro-batches.
-bool enqueue_sliced(Context &c, pulpnn_net *net, const uint8_t *input, uint8_t *stage, uint8_t *dout, int n, int n_layers)
+bool enqueue_sliced(Context &c, pulpnn_net *net, const uint8_t *input, uint8_t *stage, uint8_t *dout, int n, int n_layers,
+                    bool pipelined)
 {
   const int micro = net->micro > 0 ? net->micro : n;
   int sizes[64];
   int n_slices = 0;
   {
-    const int want = 4;        // measured at batch 1024: 5 slices lose 2 %, 6 lose 5 %, 8 lose 7 %
+    // Every slice walks all layers: some 4 us each before the first image counts. A slice is worth it while its copy
+    // (55 GB/s) takes about twice that, up to four (measured at batch 1024: 5 slices lose 2 %, 6 lose 5 %, 8 lose 7 %).
+    // Pipelined batches overlap their copies with one another's compute already: half as many. MobileNetV1, us per
+    // batch, four slices / as chosen here: blocking calls at batch 8 473 / 178, 64 643 / 457, 128 852 / 706, 256 1219 /
+    // 1122; pipelined ones 447 / 132, 572 / 266, 743 / SL128, 1010 / SL256.
+    const double slice_bytes = (pipelined ? 4 : 2) * 4.0 * n_layers * 55e3;
+    const double fit = (double)n * net->layers.front().in_bytes / slice_bytes;
+    const int want = fit < 1.5 ? 1 : (fit < 2.5 ? 2 : (fit < 3.5 ? 3 : 4));
     const int part = (n + want - 1) / want;
     int slice = micro < part ? micro : part;
     while (slice < n && slice * want < n) slice += micro;
@@ -317,7 +325,7 @@ int run_impl(pulpnn_net *net, const uint8_t *input, void *output, int n, int n_l
     // The copy is the longer of the two (154 MB of images take longer to cross PCIe than to classify),
     // so what the overlap inside one call cannot hide is the compute of the last slice; equal slices
     // measured best. pulpnn_net_submit / pulpnn_net_wait hide that too, under the next batch's copy.
-    if (!enqueue_sliced(c, net, input, net->stage_in, dout, n, n_layers)) return c.err;
+    if (!enqueue_sliced(c, net, input, net->stage_in, dout, n, n_layers, false)) return c.err;
   }
   net->launches_last_run = thread_launch_count() - launches0;
   if (!out_dev) {
@@ -506,7 +514,7 @@ int pulpnn_net_submit(pulpnn_net_t *net, const uint8_t *input, void *output, int
     cudaStreamWaitEvent(c.stream, net->ev_out[b], 0);
   }
   const unsigned long long launches0 = thread_launch_count();
-  if (!enqueue_sliced(c, net, input, net->slot_in[b], net->slot_out[b], n_images, nl)) return -c.err;
+  if (!enqueue_sliced(c, net, input, net->slot_in[b], net->slot_out[b], n_images, nl, true)) return -c.err;
   net->launches_last_run = thread_launch_count() - launches0;
   cudaEventRecord(net->ev_compute[b], c.stream);
   cudaStreamWaitEvent(net->out_stream, net->ev_compute[b], 0);
