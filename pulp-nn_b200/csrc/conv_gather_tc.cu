@@ -45,7 +45,7 @@ constexpr int ST_G_EMPTY = 0x1000, ST_G_FULL = 0x2000;
 
 struct GatherParams {
   ConvProblem p;
-  FastDiv by_pixels, by_wo, by_chunks, by_cols;   // Ho*Wo, Wo, run_chunks; columns or pieces of a tile's row
+  FastDiv by_pixels, by_wo, by_chunks, by_cols;   // Ho*Wo, Wo, run_chunks; 16-byte pieces of a tile's row
   int M, K;                // M = B*Ho*Wo output pixels, K = ky*kx*Cin bytes per weight row
   int run, run_chunks;     // L and Lp/16
   int chunks, slabs;       // chunks of K' in all, 128-byte slabs
@@ -275,6 +275,8 @@ __global__ void __launch_bounds__(GT, 2) conv_gather_tc_kernel(const __grid_cons
     const int quad = warp & 3;
     const int r = quad * 32 + lane;
     const int pitch = g.out_vec == 16 ? ((bn >> 4) | 1) << 4 : bn + 4;   // odd number of 16-byte pieces / words: no bank conflicts
+    // ragged rows of the only channel tile: staged as the one run of bytes that they are in memory
+    const bool linear = MODE != EPI_RAW32 && g.n_tiles == 1 && g.out_vec != 1 && p.Cout % 16 != 0;
     const uint32_t t_row = tmem + ((uint32_t)(quad * 32) << 16);
     if (!dead) {
       for (int c0 = (warp >> 2) * 32; c0 < ncols; c0 += 64) {
@@ -320,6 +322,26 @@ __global__ void __launch_bounds__(GT, 2) conv_gather_tc_kernel(const __grid_cons
             }
             w[j >> 2] = pack4_sat_u8(t[0], t[1], t[2], t[3]);
           }
+          if (linear) {
+            // bytes [from, from + len) of the tile's run: whole words shifted into place, the ends byte by byte
+            const int from_b = r * ncols + c0, len = min(32, ncols - c0);
+            const int head = -from_b & 3, n_words = len > head ? (len - head) >> 2 : 0;
+            const uint32_t at_s = smem_u32(staging) + (uint32_t)from_b;
+            unsigned last = 0;
+#pragma unroll
+            for (int j = 0; j < 9; j++) {
+              const unsigned x = __funnelshift_r(j < 8 ? w[j < 8 ? j : 7] : 0u, j < 7 ? w[j < 7 ? j + 1 : 7] : 0u, 8 * head);
+              if (j < n_words) asm volatile("st.shared.b32 [%0], %1;" ::"r"(at_s + head + 4 * j), "r"(x) : "memory");
+              if (j == n_words) last = x;
+            }
+            const int tail = len > head ? (len - head) & 3 : 0;
+#pragma unroll
+            for (int b = 0; b < 3; b++) {
+              if (b < min(head, len)) asm volatile("st.shared.b8 [%0], %1;" ::"r"(at_s + b), "r"(w[0] >> (8 * b)) : "memory");
+              if (b < tail) asm volatile("st.shared.b8 [%0], %1;" ::"r"(at_s + len - tail + b), "r"(last >> (8 * b)) : "memory");
+            }
+            continue;
+          }
           uint8_t *row = staging + r * pitch + c0;
           // bn is a multiple of 16: a chunk is 16 or 32 columns of the tile
           if (g.out_vec == 16) {
@@ -346,27 +368,18 @@ __global__ void __launch_bounds__(GT, 2) conv_gather_tc_kernel(const __grid_cons
             const int rr = ncols == bn ? g.by_cols.div(i) : i / per, c = i - rr * per;
             *reinterpret_cast<uint4 *>(out + (size_t)rr * p.Cout + 16 * c) = *reinterpret_cast<const uint4 *>(staging + rr * pitch + 16 * c);
           }
-        } else if (g.n_tiles == 1 && g.out_vec >= 4) {
-          // the tile is one contiguous run of rows * N bytes (its start a multiple of 128): words, wherever rows end
+        } else if (linear) {
+          // the run starts at a multiple of 128 bytes of the output
           const int total = rows * ncols;
-          for (int i = tid; i < total >> 2; i += GT) {
-            const int o = 4 * i;
-            int rr = g.by_cols.div(o), c = o - rr * ncols;
-            unsigned v;
-            if (c + 4 <= ncols) {
-              const unsigned *s4 = reinterpret_cast<const unsigned *>(staging + rr * pitch + (c & ~3));
-              v = __funnelshift_r(s4[0], s4[1], (c & 3) * 8);
-            } else {
-              v = 0;
-#pragma unroll
-              for (int b = 0; b < 4; b++) {
-                v |= (unsigned)staging[rr * pitch + c] << (8 * b);
-                if (++c == ncols) { c = 0; rr++; }
-              }
-            }
-            *reinterpret_cast<unsigned *>(out + o) = v;
+          int done;
+          if ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0) {
+            done = total & ~15;
+            for (int o = 16 * tid; o < done; o += 16 * GT) *reinterpret_cast<uint4 *>(out + o) = *reinterpret_cast<const uint4 *>(staging + o);
+          } else {
+            done = total & ~3;
+            for (int o = 4 * tid; o < done; o += 4 * GT) *reinterpret_cast<unsigned *>(out + o) = *reinterpret_cast<const unsigned *>(staging + o);
           }
-          for (int o = (total & ~3) + tid; o < total; o += GT) out[o] = staging[(o / ncols) * pitch + o % ncols];
+          for (int o = done + tid; o < total; o += GT) out[o] = staging[o];
         } else if (g.out_vec >= 4 && p.Cout % 4 == 0) {
           const int per = ncols >> 2;
           for (int i = tid; i < rows * per; i += GT) {
@@ -479,8 +492,7 @@ bool launch_conv_gather_tc(Context &c, const ConvProblem &p)
   const uintptr_t out_a = reinterpret_cast<uintptr_t>(p.out);
   g.out_vec = (p.Cout % 16 == 0 && (out_a & 15) == 0) ? 16 : ((out_a & 3) == 0 ? 4 : 1);
 
-  // the divisor of the copy-out: 16-byte pieces of a full tile's row, or columns of the only tile
-  g.by_cols.set((unsigned)(p.Cout % 16 == 0 && g.out_vec == 16 ? g.bn / 16 : p.Cout));
+  g.by_cols.set((unsigned)(g.bn / 16));              // 16-byte pieces of a full tile's row
 
   // two CTAs per SM: the ring (at least three stages, which also hold the output tile) and, if it fits, all of W
   const int half_sm = SMEM_SM / 2 - STATIC_SMEM - SMEM_RESERVED - 1024;

@@ -260,7 +260,7 @@ bool enqueue_sliced(Context &c, pulpnn_net *net, const uint8_t *input, uint8_t *
     // (55 GB/s) takes about twice that, up to four (measured at batch 1024: 5 slices lose 2 %, 6 lose 5 %, 8 lose 7 %).
     // Pipelined batches overlap their copies with one another's compute already: half as many. MobileNetV1, us per
     // batch, four slices / as chosen here: blocking calls at batch 8 473 / 178, 64 643 / 457, 128 852 / 706, 256 1219 /
-    // 1122; pipelined ones 447 / 132, 572 / 266, 743 / SL128, 1010 / SL256.
+    // 1122; pipelined ones 447 / 132, 572 / 266, 743 / 389, 1010 / 731.
     const double slice_bytes = (pipelined ? 4 : 2) * 4.0 * n_layers * 55e3;
     const double fit = (double)n * net->layers.front().in_bytes / slice_bytes;
     const int want = fit < 1.5 ? 1 : (fit < 2.5 ? 2 : (fit < 3.5 ? 3 : 4));
