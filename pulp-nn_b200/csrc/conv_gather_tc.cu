@@ -46,6 +46,7 @@ constexpr int ST_G_EMPTY = 0x1000, ST_G_FULL = 0x2000;
 struct GatherParams {
   ConvProblem p;
   FastDiv by_pixels, by_wo, by_chunks, by_cols;   // Ho*Wo, Wo, run_chunks; 16-byte pieces of a tile's row
+  FastDiv by_bn, by_last;                         // columns of a tile, of the last one
   int M, K;                // M = B*Ho*Wo output pixels, K = ky*kx*Cin bytes per weight row
   int run, run_chunks;     // L and Lp/16
   int chunks, slabs;       // chunks of K' in all, 128-byte slabs
@@ -387,8 +388,19 @@ __global__ void __launch_bounds__(GT, 2) conv_gather_tc_kernel(const __grid_cons
             *reinterpret_cast<unsigned *>(out + (size_t)rr * p.Cout + 4 * c) = *reinterpret_cast<const unsigned *>(staging + rr * pitch + 4 * c);
           }
         } else {
-          for (int rr = warp; rr < rows; rr += GT / 32)
-            for (int c = lane; c < ncols; c += 32) out[(size_t)rr * p.Cout + c] = staging[rr * pitch + c];
+          // byte by byte: a warp to a row while that fills its lanes
+          if (ncols >= 64) {
+#pragma unroll 2
+            for (int rr = warp; rr < rows; rr += GT / 32)
+              for (int c = lane; c < ncols; c += 32) out[(size_t)rr * p.Cout + c] = staging[rr * pitch + c];
+          } else {
+            const FastDiv &by = nt == g.n_tiles - 1 ? g.by_last : g.by_bn;
+#pragma unroll 4
+            for (int i = tid; i < rows * ncols; i += GT) {
+              const int rr = by.div(i), c = i - rr * ncols;
+              out[(size_t)rr * p.Cout + c] = staging[rr * pitch + c];
+            }
+          }
         }
       }
     }
@@ -470,6 +482,8 @@ bool launch_conv_gather_tc(Context &c, const ConvProblem &p)
   // How many ways to cut the channels (bn = 16 .. 256) and the reduction (1 .. 8 CTAs of a cluster): the
   // cheapest count of gathered rows on the busiest SM's pair of CTAs. A tile's set-up, drain and stores
   // weigh about 300 rows, the exchange through the cluster 150 more; at least two slabs per CTA.
+  // Rows of no whole words in several tiles leave byte by byte.
+  const bool bytewise = p.epi.mode != EPI_RAW32 && (p.Cout % 4 != 0 || (reinterpret_cast<uintptr_t>(p.out) & 3));
   long long best = -1;
   for (int split = 1; split <= 8; split *= 2) {
     const int per = (g.slabs + split - 1) / split;
@@ -479,7 +493,7 @@ bool launch_conv_gather_tc(Context &c, const ConvProblem &p)
       const int bn = ((p.Cout + want - 1) / want + 15) & ~15, nt = (p.Cout + bn - 1) / bn;
       if (split > 1 && bn > 64) continue;              // the partial sums have to fit the ring
       const long long rounds = ((long long)g.m_tiles * nt * split + 2 * sms - 1) / (2 * sms);
-      const long long cost = rounds * ((long long)per * (GBM + bn) + 300 + (split > 1 ? 150 : 0));
+      const long long cost = rounds * ((long long)per * (GBM + bn) + 300 + (split > 1 ? 150 : 0) + (bytewise && nt > 1 && split == 1 ? 100 + bn : 0));
       if (best < 0 || cost < best) { best = cost; g.bn = bn; g.n_tiles = nt; g.k_split = split; g.slabs_per = per; }
       if (bn == 16) break;
     }
@@ -492,6 +506,8 @@ bool launch_conv_gather_tc(Context &c, const ConvProblem &p)
   const uintptr_t out_a = reinterpret_cast<uintptr_t>(p.out);
   g.out_vec = (p.Cout % 16 == 0 && (out_a & 15) == 0) ? 16 : ((out_a & 3) == 0 ? 4 : 1);
 
+  g.by_bn.set((unsigned)g.bn);
+  g.by_last.set((unsigned)(p.Cout - (g.n_tiles - 1) * g.bn));
   g.by_cols.set((unsigned)(g.bn / 16));              // 16-byte pieces of a full tile's row
 
   // two CTAs per SM: the ring (at least three stages, which also hold the output tile) and, if it fits, all of W
