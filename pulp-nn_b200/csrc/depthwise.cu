@@ -263,18 +263,21 @@ bool launch_dw_mode(Context &c, const DepthwiseProblem &p)
 
 // The plane-staging kernel has the shortest start, the TMA kernels and the one that keeps its rows in registers the
 // higher rate. Where the lines lie (bytes read and written; us planes / other kernel):
-//  HWC, TMA:   1x28x28x256 0.4 MB 2.4 / 5.4, 8x28x28x256 3.2 MB 5.0 / 5.5, 16x28x28x256 6.4 MB 7.0 / 5.5 -- wide images;
-//              8x14x14x512 1.6 MB 4.0 / 4.2, 16x14x14x512 3.2 MB 5.1 / 4.2; 1x7x7x1024 0.1 MB 2.3 / 2.9, 8x7x7x1024
-//              0.8 MB 3.3 / 2.9: the smaller the image, the shorter the TMA kernel's strips
-//  HWC, registers: 8x56x56x100 5.0 MB 7.3 / 8.3, 16x56x56x100 10 MB 11.3 / 9.6; stride 2: 6.3 MB 8.1 / 11.8, 12.5 MB 13.0 / 11.8
-//  CHW, TMA:   16x32x32x128 4.2 MB 6.2 / 7.3, 8x112x112x32 6.4 MB 8.2 / 7.8
+//  HWC, TMA:   8x28x28x256 3.2 MB 4.2 / 5.5, 16x28x28x256 6.4 MB 6.0 / 5.5; 8x14x14x512 1.6 MB 3.5 / 4.2, 16x14x14x512
+//              3.2 MB 4.4 / 4.2; 4x7x7x1024 0.4 MB 2.3 / 2.9, 8x7x7x1024 0.8 MB 3.0 / 2.9 (the smaller the image, the
+//              shorter the TMA kernel's strips); stride 2: 16x28x28x256 4.0 MB 4.2 / 5.3, 24 of them 6.0 MB 5.8 / 5.3,
+//              16x14x14x512 2.0 MB 3.2 / 3.4
+//  HWC, registers: 32x56x56x24 4.8 MB 6.3 / 8.2, 16x56x56x100 10 MB 9.6 / 9.7, 64x56x56x24 9.6 MB 9.6 / 9.5; stride 2:
+//              32x56x56x100 12.5 MB 8.3 / 11.8
+//  CHW, TMA:   16x32x32x128 4.2 MB 5.9 / 7.4, 8x112x112x32 6.4 MB 7.5 / 7.8; stride 2: 4x112x112x64 4.0 MB 5.4 / 6.7, 8 of
+//              them 8.0 MB 8.3 / 6.6
 static bool planes_first(const DepthwiseProblem &p, bool tma)
 {
   const long long bytes = (long long)p.B * p.C * ((long long)p.H * p.W + (long long)p.Ho * p.Wo);
   long long kb;
-  if (!p.in_is_hwc) kb = 4500;
-  else if (tma)     kb = p.Wo >= 28 ? 3300 : (p.Wo >= 14 ? 1700 : 400);
-  else              kb = p.sx == 1 ? 6000 : 9000;
+  if (!p.in_is_hwc) kb = p.sx == 1 ? 6500 : 4500;
+  else if (tma)     kb = p.H >= 28 ? 4500 : (p.H >= 14 ? 2200 : 600);
+  else              kb = p.sx == 1 ? 9000 : 16000;
   return bytes <= kb * 1000;
 }
 

@@ -10,11 +10,13 @@
 // one or two dp4a per output against copies of its taps shifted to the byte the window starts at -- no
 // unpacking and no funnel shifts. Each plane row is read once for the R rows it feeds.
 //
-// What bounds it: instruction issue -- a warp of 5x5 outputs costs some 25 instructions in the dp4a and
-// the requantised byte stores, about as many again to stage its share of the input (halo included) and to
-// set the CTA up. Measured (us, graph replay, before / after): 28x28x120 5x5 HWC at batch 32 39.3 / 10.9, the
-// same from CHW 97.8 / 11.3, 14x14x475 5x5 stride 2 at batch 20 15.9 / 6.1, 56x56x61 3x3 at batch 8 25.5 /
-// 5.7, 30x30x64 3x3 CHW at batch 64 70.9 / 8.9.
+// What bounds it: instruction issue -- a warp of 3x3 outputs costs some 12 instructions in the dp4a and
+// the requantised byte stores and about as many again to stage its share of the input, halo included (64 % of
+// the issue slots taken on 70x70x187). So a filter row is expanded once per CTA and not per warp, offsets are
+// 32 bits, and pixels that lie across words are two word loads and a funnel shift. Measured (us, graph replay;
+// the kernels it replaces / now): 28x28x120 5x5 HWC at batch 32 39.3 / 8.8, the same from CHW 97.8 / 9.9,
+// 14x14x475 5x5 stride 2 at batch 20 15.9 / 5.6, 56x56x61 3x3 at batch 8 25.5 / 4.7, 30x30x64 3x3 CHW at batch
+// 64 70.9 / 8.4, 70x70x187 3x3 at batch 32 458 / 33.7.
 #include "internal.cuh"
 #include "unaligned16.cuh"
 
@@ -31,6 +33,7 @@ struct PlanesParams {
   int plane;                    // bytes of a plane, an odd number of words
   int words;                    // HWC: channels in whole aligned words
   int quads;                    // groups of four output columns
+  FastDiv by_groups, by_bands;
   FastDiv by_qw, by_per, by_quads;   // words (CHW: 16-byte pieces) of a plane row, of a plane; quads
 };
 
@@ -50,10 +53,8 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
   extern __shared__ __align__(16) uint8_t planes[];
   const DepthwiseProblem &p = g.p;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  unsigned blk = blockIdx.x;
-  const int grp = (int)(blk % (unsigned)g.groups); blk /= (unsigned)g.groups;
-  const int band = (int)(blk % (unsigned)g.bands);
-  const int b = (int)(blk / (unsigned)g.bands);
+  const int t0 = g.by_groups.div((int)blockIdx.x), grp = (int)blockIdx.x - t0 * g.groups;
+  const int b = g.by_bands.div(t0), band = t0 - b * g.bands;
   const int c0 = grp * CG, nch = min(CG, p.C - c0);
   const int oy0 = band * g.band;
   const int iy0 = oy0 * S - p.pt;
@@ -62,38 +63,81 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
   pdl_wait();
   pdl_launch_dependents();
 
+  // what the compute phase needs of the parameters is on its way while the rows are staged: a filter row of one
+  // channel per thread, the lane's channel's requantisation
+  const Epilogue &e = p.epi;
+  const int cl = lane % CG, sub = lane / CG;
+  const int c = c0 + min(cl, nch - 1);
+  long long kk = 0, ll = 0;
+  if (MODE == EPI_BN32) {
+    kk = __ldg(reinterpret_cast<const int *>(e.k) + c);
+    ll = __ldg(reinterpret_cast<const int *>(e.lambda) + c);
+  } else if (MODE == EPI_BN64) {
+    kk = __ldg(reinterpret_cast<const long long *>(e.k) + c);
+    ll = __ldg(reinterpret_cast<const long long *>(e.lambda) + c);
+  }
+  const int bias = e.bias ? (int)__ldg(reinterpret_cast<const int8_t *>(e.bias) + c) : 0;
+  static_assert(K * CG <= DT, "a filter row per thread");
+  const int wc = tid % CG, wfy = tid / CG;
+  unsigned taps[K];
+#pragma unroll
+  for (int fx = 0; fx < K; fx++)
+    taps[fx] = wfy < K && wc < nch ? (unsigned)(uint8_t)__ldg(p.w + ((size_t)(c0 + wc) * K + wfy) * K + fx) : 0u;
+
   // ---- stage the planes -----------------------------------------------------------------------
   if (p.in_is_hwc) {
     constexpr int CQ = CG / 4;
-    const uint8_t *img = p.in + (size_t)b * p.H * p.W * p.C + c0;
+    // 32-bit offsets into the image from the word at or below its first byte; the words that lie inside the tensor
+    const size_t off = (size_t)b * p.H * p.W * p.C;
+    const int lead = (int)(reinterpret_cast<uintptr_t>(p.in + off) & 3);
+    const uint8_t *img = p.in + off - lead;
+    const int lo = b > 0 ? -64 : lead, hi = lead + p.H * p.W * p.C + (b < p.B - 1 ? 64 : 0);
     const int items = g.rows_in * qw;                       // words of four pixels, the thread's four channels
     const int cq = tid % CQ, left = nch - 4 * cq;           // channels of this word that exist
     constexpr int STEP = DT / CQ;
     constexpr int U = 2;                                    // items of a thread in flight
     for (int it0 = tid / CQ; it0 < items; it0 += U * STEP) {
-      unsigned v[U][4];
-      int dst[U];
+      unsigned v[U][4], v1[U][4];
+      int dst[U], at[U];
 #pragma unroll
       for (int u = 0; u < U; u++) {
         const int it = it0 + u * STEP;
         const int row = g.by_qw.div(it), q = it - row * qw;
-        const int iy = iy0 + row;
+        const int iy = iy0 + row, ix = 4 * q - p.pl;
         const bool ok = it < items && (unsigned)iy < (unsigned)p.H && left > 0;
-        const int ix = 4 * q - p.pl;
-        const uint8_t *src = img + ((size_t)(ok ? iy : 0) * p.W + ix) * p.C + 4 * cq;
+        at[u] = (iy * p.W + ix) * p.C + c0 + 4 * cq + lead;
         dst[u] = it < items ? 4 * cq * g.plane + row * g.row_pitch + 4 * q : -1;
         if (g.words) {
 #pragma unroll
-          for (int i = 0; i < 4; i++) v[u][i] = ldg4_if(src + (size_t)i * p.C, ok && (unsigned)(ix + i) < (unsigned)p.W);
-        } else {
+          for (int i = 0; i < 4; i++) v[u][i] = ldg4_if(img + at[u] + i * p.C, ok && (unsigned)(ix + i) < (unsigned)p.W);
+        } else if (!ok || ((at[u] & ~3) >= lo && at[u] + 3 * p.C + 8 <= hi)) {
 #pragma unroll
           for (int i = 0; i < 4; i++) {
             const bool in = ok && (unsigned)(ix + i) < (unsigned)p.W;
-            v[u][i] = 0;
+            const uint8_t *w = img + ((at[u] + i * p.C) & ~3);
+            v[u][i] = ldg4_if(w, in);
+            v1[u][i] = ldg4_if(w + 4, in);
+          }
+        } else {
+          // the ends of the tensor: byte by byte, put where the shift takes them
 #pragma unroll
-            for (int k = 0; k < 4; k++) v[u][i] |= ldg1_if(src + (size_t)i * p.C + k, in && k < left) << (8 * k);
+          for (int i = 0; i < 4; i++) {
+            const int o = at[u] + i * p.C;
+            const bool in = (unsigned)(ix + i) < (unsigned)p.W;
+            unsigned x = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) x |= ldg1_if(img + o + k, in && k < left) << (8 * k);
+            const unsigned sh = (unsigned)(o & 3) * 8;
+            v[u][i] = x << sh;
+            v1[u][i] = sh ? x >> (32 - sh) : 0;
           }
         }
+      }
+      if (!g.words) {
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) v[u][i] = __funnelshift_r(v[u][i], v1[u][i], (unsigned)(at[u] + i * p.C) * 8);
       }
 #pragma unroll
       for (int u = 0; u < U; u++) {
@@ -145,39 +189,41 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
     }
   }
 
-  // ---- this lane's channel: shifted copies of its filter rows, requantisation parameters -----------
-  const int cl = lane % CG, sub = lane / CG;
-  const int c = c0 + min(cl, nch - 1);
-  unsigned wv[K][NV][2];
-#pragma unroll
-  for (int fy = 0; fy < K; fy++) {
+  // ---- the filter rows shifted to every window start, [row][start][word][channel] ------------------
+  unsigned *wsm = reinterpret_cast<unsigned *>(planes + CG * g.plane);
+  if (wfy < K) {
     unsigned long long t = 0;
 #pragma unroll
-    for (int fx = 0; fx < K; fx++)
-      t |= (unsigned long long)(uint8_t)__ldg(p.w + ((size_t)c * K + fy) * K + fx) << (8 * fx);
+    for (int fx = 0; fx < K; fx++) t |= (unsigned long long)taps[fx] << (8 * fx);
 #pragma unroll
     for (int v = 0; v < NV; v++) {
-      wv[fy][v][0] = (unsigned)(t << (8 * v * S));
-      wv[fy][v][1] = (unsigned)((t << (8 * v * S)) >> 32);
+      wsm[((wfy * NV + v) * 2 + 0) * CG + wc] = (unsigned)(t << (8 * v * S));
+      wsm[((wfy * NV + v) * 2 + 1) * CG + wc] = (unsigned)((t << (8 * v * S)) >> 32);
     }
   }
-  const Epilogue &e = p.epi;
-  long long kk = 0, ll = 0;
-  if (MODE == EPI_BN32) {
-    kk = __ldg(reinterpret_cast<const int *>(e.k) + c);
-    ll = __ldg(reinterpret_cast<const int *>(e.lambda) + c);
-  } else if (MODE == EPI_BN64) {
-    kk = __ldg(reinterpret_cast<const long long *>(e.k) + c);
-    ll = __ldg(reinterpret_cast<const long long *>(e.lambda) + c);
-  }
-  const int bias = e.bias ? (int)__ldg(reinterpret_cast<const int8_t *>(e.bias) + c) : 0;
   const bool fits = MODE == EPI_BN64 && __all_sync(0xffffffffu, bn_fits_32(kk, ll, K * K * ACC_PER_TERM + 128, e.shift));
   __syncthreads();
+  unsigned wv[K][NV][2];
+#pragma unroll
+  for (int fy = 0; fy < K; fy++)
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      wv[fy][v][0] = wsm[((fy * NV + v) * 2 + 0) * CG + cl];
+      wv[fy][v][1] = wsm[((fy * NV + v) * 2 + 1) * CG + cl];
+    }
+  // the shifted value before it is cut to a byte
+  auto scaled = [&](int a) {
+    if (MODE == EPI_BN32 || fits) return (int)((unsigned)(int)kk * (unsigned)a + (unsigned)(int)ll) >> e.shift;
+    if (MODE == EPI_BN64) return (int)((long long)((unsigned long long)kk * (unsigned long long)(long long)a + (unsigned long long)ll) >> e.shift);
+    if (MODE == EPI_MULT) return (int)(short)((int)((unsigned)e.out_mult * (unsigned)a) >> e.shift);
+    return a >> e.shift;
+  };
 
   // ---- compute: a unit is four columns x R rows of the warp's channels ------------------------------
   const int rows = min(g.band, p.Ho - oy0);
   const int units = ((rows + R - 1) / R) * g.quads;
   const uint8_t *mine = planes + (size_t)cl * g.plane;
+  uint8_t *out = p.out + (size_t)b * p.Ho * p.Wo * p.C;
   for (int u = warp * (32 / CG) + sub; u < units; u += (DT / 32) * (32 / CG)) {
     const int rb = g.by_quads.div(u), xq = u - rb * g.quads;
     int acc[R][4];
@@ -203,16 +249,21 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
         }
       }
     }
-    if (cl < nch) {
-      const int oy = oy0 + rb * R, ox = xq * 4;
-      uint8_t *o = p.out + (((size_t)b * p.Ho + oy) * p.Wo + ox) * p.C + c;
+    const int oy = oy0 + rb * R, ox = xq * 4;
+    const bool whole = ox + 4 <= p.Wo;
+    unsigned o = (unsigned)((oy * p.Wo + ox) * p.C + c);
 #pragma unroll
-      for (int r = 0; r < R; r++) {
-        if (oy + r >= p.Ho) break;
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-          if (ox + i < p.Wo) o[((size_t)r * p.Wo + i) * p.C] = (uint8_t)(fits ? requant_kl<EPI_BN32>(acc[r][i], kk, ll, e.out_mult, e.shift)
-                                                            : requant_kl<MODE>(acc[r][i], kk, ll, e.out_mult, e.shift));
+    for (int r = 0; r < R; r++, o += (unsigned)(p.Wo * p.C)) {
+      const unsigned w = pack4_sat_u8(scaled(acc[r][0]), scaled(acc[r][1]), scaled(acc[r][2]), scaled(acc[r][3]));
+      if (cl >= nch || oy + r >= p.Ho) continue;
+      out[o] = (uint8_t)w;
+      if (whole) {
+        out[o + p.C] = (uint8_t)(w >> 8);
+        out[o + 2 * p.C] = (uint8_t)(w >> 16);
+        out[o + 3 * p.C] = (uint8_t)(w >> 24);
+      } else {
+        if (ox + 1 < p.Wo) out[o + p.C] = (uint8_t)(w >> 8);
+        if (ox + 2 < p.Wo) out[o + 2 * p.C] = (uint8_t)(w >> 16);
       }
     }
   }
@@ -270,12 +321,15 @@ bool configure(const DepthwiseProblem &p, int sms, PlanesParams &g, int &cg, int
   if (plane_of(g.band) * cg > 200 * 1024) return false;
   // 32-bit offsets inside a group of channels, the rows above and below its image included
   if (((long long)cg * p.H + p.pt + g.band * S + K) * p.W > 0x7fff0000LL) return false;
+  if ((long long)p.Ho * p.Wo * p.C > 0x7fff0000LL || ((long long)p.H + p.pt + g.band * S + K) * p.W * p.C > 0x7fff0000LL) return false;
   g.bands = (p.Ho + g.band - 1) / g.band;
   if ((long long)g.groups * g.bands * p.B > 0x7fffffffLL) return false;
   g.row_pitch = (int)pitch;
   g.rows_in = (g.band - 1) * S + K;
   g.plane = (int)plane_of(g.band);
-  smem = g.plane * cg;
+  smem = g.plane * cg + K * (4 / S) * 2 * cg * 4;
+  g.by_groups.set((unsigned)g.groups);
+  g.by_bands.set((unsigned)g.bands);
   const int piece = p.in_is_hwc ? 4 : 16;
   g.by_qw.set((unsigned)(g.row_pitch / piece));
   g.by_per.set((unsigned)(g.rows_in * (g.row_pitch / piece)));
