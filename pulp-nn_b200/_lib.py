@@ -27,7 +27,8 @@ CU_SOURCES = ["context.cu", "conv_generic.cu", "depthwise.cu", "pool_add.cu", "e
               "igemm_tc.cu", "net.cu", "depthwise_hwc3x3.cu",
               "conv_smallcin.cu", "depthwise_hwc3x3_tma.cu",
               "conv_smallcin_tc.cu", "layout.cu", "subbyte.cu", "diagnostics.cu", "dwpw_fused.cu", "igemm_tc2.cu", "gemm_fewrows.cu", "dwpw_tcdw.cu",
-              "conv_gather_tc.cu", "depthwise_planes.cu", "packed_calls.cu", "igemm_split.cu"]
+              "conv_gather_tc.cu", "depthwise_planes.cu", "packed_calls.cu", "igemm_split.cu",
+              "conv_halo_tc.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC"]
 

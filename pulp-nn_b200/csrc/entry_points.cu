@@ -473,6 +473,7 @@ static bool gather_first(const Context &c, const ConvProblem &p)
 
 bool launch_conv(Context &c, const ConvProblem &p)
 {
+  if (!c.opt_force_generic && c.opt_split_k == 0 && !(c.opt_tune & 64) && conv_halo_tc_supported(c, p)) return launch_conv_halo_tc(c, p);
   switch (few_tiles_form(c, p)) {
     case FewTiles::rows: return launch_gemm_fewrows(c, p);
     case FewTiles::gather: return launch_conv_gather_tc(c, p);

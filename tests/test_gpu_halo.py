@@ -1,0 +1,54 @@
+"""The convolution kernel that fetches every input pixel once per tile, against the CPU checker, byte for byte: every
+requantisation mode, both slab widths, several channel chunks and tiles, patches that cross every edge of the image,
+kernels that are not square, weights of one and of several channel tiles, few and many tiles per CTA."""
+import pytest
+
+from conftest import pulpnn
+from test_gpu_parity import MODES, conv_kw, same
+
+pytestmark = pytest.mark.gpu
+api, wl = pulpnn.api, pulpnn.workloads
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    return pulpnn.GpuKernels(host_buffers=False)
+
+
+@pytest.fixture(autouse=True)
+def _status():
+    yield
+    assert api.device_status() == 0
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("relu,bn", MODES)
+def test_modes(bits, relu, bn, gpu, restatement):
+    c = wl.conv_case(110, 28, 28, 64, 64, batch=40, bits=bits, out_shift=11, with_bias=True, out_mult=3, relu=relu, bn=bn,
+                     w_range=(-128, 127), k_range=(-64, 64), lam_range=(-2 ** 20, 2 ** 20))
+    got = gpu.conv(bits, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c))
+    c["x"] = c["x"][-1:]
+    same(got[-1:], restatement.conv(bits, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
+
+
+@pytest.mark.parametrize("H,W,Cin,Cout,kernel,pads,batch", [
+    (28, 28, 128, 128, (3, 3), (1, 1, 1, 1), 32),
+    (16, 8, 128, 128, (3, 3), (1, 1, 1, 1), 160),        # a patch is an image
+    (33, 17, 64, 80, (3, 3), (1, 1, 1, 1), 60),           # ragged patches, columns that are no power of two
+    (30, 31, 64, 16, (5, 5), (2, 2, 2, 2), 40),
+    (20, 40, 128, 48, (3, 1), (1, 1, 0, 0), 40),
+    (20, 40, 64, 64, (1, 7), (0, 0, 3, 3), 40),
+    (40, 24, 64, 64, (3, 3), (0, 2, 2, 0), 50),
+    (24, 24, 128, 256, (3, 3), (1, 1, 1, 1), 40),         # two channel tiles
+    (16, 24, 256, 64, (3, 3), (1, 1, 1, 1), 80),          # two chunks
+    (16, 24, 192, 96, (3, 3), (1, 1, 1, 1), 80),          # three chunks of 64
+    (28, 28, 32, 64, (3, 3), (1, 1, 1, 1), 40),           # slabs of 32 bytes
+    (17, 30, 96, 112, (3, 3), (1, 1, 1, 1), 40),
+])
+@pytest.mark.parametrize("strides", [(1, 1), (2, 2), (2, 1), (1, 2)])
+def test_shapes(H, W, Cin, Cout, kernel, pads, batch, strides, gpu, restatement):
+    c = wl.conv_case(111, H, W, Cin, Cout, kernel=kernel, pads=pads, strides=strides, batch=batch, out_shift=12)
+    got = gpu.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c))
+    x = c["x"]
+    for b in (0, batch // 2, batch - 1):
+        same(got[b:b + 1], restatement.conv(32, x[b:b + 1], c["w"], c["k"], c["lam"], **conv_kw(c)))
