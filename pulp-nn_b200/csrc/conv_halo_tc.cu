@@ -1,5 +1,5 @@
-// conv_halo_tc.cu -- stride-1 spatial convolution on the tensor cores with every input pixel fetched ONCE per
-// tile (arithmetic of igemm_tc.cu; 32bit/src/pulp_nn_conv_Ho_parallel.c:80-249).
+// conv_halo_tc.cu -- spatial convolution, strides 1 and 2, on the tensor cores with every input pixel fetched ONCE
+// per tile (arithmetic of igemm_tc.cu; 32bit/src/pulp_nn_conv_Ho_parallel.c:80-249).
 //
 // igemm_tc.cu fetches a tile's operand tap by tap: nine TMA boxes of the same pixels for a 3x3 kernel, and with
 // the weights streamed beside them that traffic into the SM is what its convolutions wait for. Here a tile is a
@@ -10,8 +10,8 @@
 // address for TMA and MMA alike, so a shifted start needs nothing else. The CTA's slice of W stays in shared
 // memory for its lifetime; a 128-channel 3x3 tile then takes 23 KB from L2 instead of 295.
 //
-// Roles of a CTA (persistent, 10 warps): warp 0 TMA, warp 1 MMA issue, warps 2..9 epilogue (two accumulators
-// in tensor memory; requantised bytes through a staging tile, out in 16-byte pieces).
+// Roles of a CTA (persistent, 18 warps): warp 0 TMA, warp 1 MMA issue, warps 2..17 four epilogue groups that take the
+// tiles in turn from a ring of accumulators in tensor memory and store the requantised rows from registers.
 //
 // What bounds it: the MMAs -- one costs some 80 cycles, bound by reading 32 bytes of each of its rows, so the issuing
 // thread adds a tabled offset per tap and nothing else (with the offsets computed there a tap of one MMA took 270
@@ -202,31 +202,8 @@ conv_halo_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         uint32_t v[32];
         tmem_ld_32(t_row + (uint32_t)c0, v);
         tmem_wait_ld();
-        const bool fits = MODE == EPI_BN64 &&
-            __all_sync(0xffffffffu, c0 + lane >= ncols || bn_fits_32(par_k[c0 + lane], par_l[c0 + lane], acc_bound(g.K), e.shift));
         unsigned w[8];
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          int t[4];
-          // columns past the last channel read stale parameters; their bytes are never stored
-          if (MODE == EPI_BN32) {
-            const int4 kk = *reinterpret_cast<const int4 *>(reinterpret_cast<const int *>(par_k) + c0 + j);
-            const int4 ll = *reinterpret_cast<const int4 *>(reinterpret_cast<const int *>(par_l) + c0 + j);
-            t[0] = (int)((unsigned)kk.x * v[j] + (unsigned)ll.x) >> e.shift;
-            t[1] = (int)((unsigned)kk.y * v[j + 1] + (unsigned)ll.y) >> e.shift;
-            t[2] = (int)((unsigned)kk.z * v[j + 2] + (unsigned)ll.z) >> e.shift;
-            t[3] = (int)((unsigned)kk.w * v[j + 3] + (unsigned)ll.w) >> e.shift;
-          } else if (MODE == EPI_BN64) {
-            requant4_bn64(par_k + c0 + j, par_l + c0 + j, v[j], v[j + 1], v[j + 2], v[j + 3], e.shift, fits, t);
-          } else {
-            const int4 bb = *reinterpret_cast<const int4 *>(reinterpret_cast<const int *>(par_l) + c0 + j);
-            const int a4[4] = {(int)v[j] + bb.x, (int)v[j + 1] + bb.y, (int)v[j + 2] + bb.z, (int)v[j + 3] + bb.w};
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-              t[u] = MODE == EPI_MULT ? (int)(short)((int)((unsigned)e.out_mult * (unsigned)a4[u]) >> e.shift) : a4[u] >> e.shift;
-          }
-          w[j >> 2] = pack4_sat_u8(t[0], t[1], t[2], t[3]);
-        }
+        requant32_cols<MODE>(v, c0, ncols, par_k, par_l, e, g.K, w);
         if (store) {
           // whole 32-byte sectors of a pixel where the channel count allows
           uint8_t *o = out + c0;
@@ -278,19 +255,19 @@ bool launch_halo_bk(Context &c, const CUtensorMap &a, const CUtensorMap &w, cons
   return launch_halo<MODE, 128>(c, a, w, g, grid, smem);
 }
 
-// Lays the problem out; false where it does not fit or another kernel is faster. The channels are cut into the
-// tiles with the least estimated time: an MMA takes 80 cycles or BN / 2, whichever is more, a row of a TMA box some 12,
+// Lays the problem out and returns the estimated ns, -1 where it does not fit or igemm_tc.cu is faster. The channels
+// are cut into the tiles with the least estimated time: an MMA takes 80 cycles or BN / 2, whichever is more, a row of a TMA box some 12,
 // the CTA's slice of W 80 bytes per ns, and the tiles come in rounds of as many as there are SMs. Cutting the channels
 // multiplies the MMAs that narrow tiles leave half idle: beyond twice those of one tile, and more than two rounds,
 // igemm_tc.cu is faster (14x14x256 -> 256 at batch 64, four tiles of 64: 17.8 us against 12.9; 28x28x224 -> 224 at
 // batch 16 19.9 / 18.3; 28x28x160 -> 160 at batch 32 18.8 / 19.1; in one or two rounds 14x14x256 at batch 32 10.8 /
 // 12.3, at batch 8 6.6 / 10.4).
-bool plan_halo(const ConvProblem &p, int sms, HaloParams &g, int &bkb, int &smem)
+double plan_halo(const ConvProblem &p, int sms, HaloParams &g, int &bkb, int &smem)
 {
   if (p.sx < 1 || p.sx > 2 || p.sy < 1 || p.sy > 2 || p.ky * p.kx < 2 || p.kx > 9 || p.ky > 9 || p.Cin % 32 != 0 || p.Cout % 16 != 0)
-    return false;
-  if (p.epi.mode == EPI_RAW32) return false;
-  if ((reinterpret_cast<uintptr_t>(p.in) | reinterpret_cast<uintptr_t>(p.w) | reinterpret_cast<uintptr_t>(p.out)) & 15) return false;
+    return -1;
+  if (p.epi.mode == EPI_RAW32) return -1;
+  if ((reinterpret_cast<uintptr_t>(p.in) | reinterpret_cast<uintptr_t>(p.w) | reinterpret_cast<uintptr_t>(p.out)) & 15) return -1;
   bkb = p.Cin % 128 == 0 ? 128 : (p.Cin % 64 == 0 ? 64 : 32);
   g.epi = p.epi; g.out = static_cast<uint8_t *>(p.out);
   g.N = p.Cout; g.K = p.ky * p.kx * p.Cin; g.Ho = p.Ho; g.Wo = p.Wo; g.pt = p.pt; g.pl = p.pl; g.ky = p.ky; g.kx = p.kx;
@@ -302,7 +279,7 @@ bool plan_halo(const ConvProblem &p, int sms, HaloParams &g, int &bkb, int &smem
   g.box_stride = p.sx * p.sy * g.box_pitch;
   g.tiles_x = (p.Wo + HTW - 1) / HTW; g.tiles_y = (p.Ho + HTH - 1) / HTH;
   const long long m_tiles = (long long)p.B * g.tiles_x * g.tiles_y;
-  if (m_tiles > 0x7fffffffLL) return false;
+  if (m_tiles > 0x7fffffffLL) return -1;
   g.m_tiles = (int)m_tiles;
   double best = -1;
   for (int nt = (p.Cout + 255) / 256;; nt++) {
@@ -322,21 +299,22 @@ bool plan_halo(const ConvProblem &p, int sms, HaloParams &g, int &bkb, int &smem
     g.n_boxes = (int)(boxes < MAX_BOXES ? boxes : MAX_BOXES);
     smem = (int)(fixed + (long long)g.n_boxes * g.box_stride);
   }
-  if (best < 0) return false;
+  if (best < 0) return -1;
   g.acc_cols = 32;
   while (g.acc_cols < g.bn) g.acc_cols *= 2;
   g.n_acc = 512 / g.acc_cols < MAX_ACC ? 512 / g.acc_cols : MAX_ACC;
   g.wide_store = p.Cout % 32 == 0 && g.bn % 32 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
-  return true;
+  return best;
 }
 
 }  // namespace
 
-bool conv_halo_tc_supported(const Context &c, const ConvProblem &p)
+double conv_halo_tc_estimate(const Context &c, const ConvProblem &p)
 {
   HaloParams g = {};
   int bkb, smem;
-  return plan_halo(p, c.sm_count > 0 ? c.sm_count : 148, g, bkb, smem) && encode_tiled_fn() != nullptr;
+  const double ns = plan_halo(p, c.sm_count > 0 ? c.sm_count : 148, g, bkb, smem);
+  return ns < 0 || !encode_tiled_fn() ? -1 : 2000 + ns;
 }
 
 bool launch_conv_halo_tc(Context &c, const ConvProblem &p)
@@ -344,7 +322,7 @@ bool launch_conv_halo_tc(Context &c, const ConvProblem &p)
   HaloParams g = {};
   int bkb = 128, smem = 0;
   const int sms = c.sm_count > 0 ? c.sm_count : 148;
-  if (!plan_halo(p, sms, g, bkb, smem)) return false;
+  if (plan_halo(p, sms, g, bkb, smem) < 0) return false;
   g.const_weights = p.folded != nullptr;
   g.by_tx.set((unsigned)g.tiles_x);
   g.by_ty.set((unsigned)g.tiles_y);

@@ -420,8 +420,8 @@ void add_entry(uint8_t *a, uint8_t *b, uint8_t *out, int m1, int m2, int out_shi
 // Which kernel takes a GEMM of few tiles: the dp4a one while a CTA's eight neurons see few rows; igemm_split where a
 // cluster shares the reduction; the gathering kernel for narrow channel slabs, whose TMA boxes of 32 or 64 bytes a
 // row cost more than gathering them; igemm_tc otherwise. Measured (us, igemm_tc / gather / split, dp4a):
-//   196 x 512 -> 512     5.4 / 5.3 / 4.6, 13.7      196 x 256 -> 512   3.8 / 4.0 / 4.7, 13.9     392 x 512 -> 512  5.5 / 6.9 / 5.7
-//   49 x 512 -> 1024     5.2 / 5.1 / 4.6,  5.0      49 x 1024 -> 1024  9.6 / 5.6 / 5.2,  6.9     196 x 1024 -> 1024  14.2 / 7.3 / 5.7
+//   196 x 512 -> 512     5.4 / 5.3 / 4.1, 13.7      196 x 256 -> 512   3.8 / 4.0 / 4.7, 13.9     392 x 512 -> 512  5.5 / 6.9 / 5.7
+//   49 x 512 -> 1024     5.2 / 5.1 / 4.2,  5.0      49 x 1024 -> 1024  9.6 / 5.6 / 5.2,  6.9     196 x 1024 -> 1024  14.2 / 7.3 / 5.7
 //   1 x 1024 -> 1000     8.2 / 5.2 / 4.9,  2.2      37 x 1024 -> 1000  9.2 / 5.6 / 5.1,  4.8     128 x 1024 -> 1000  13.2 / 5.8 / 5.2, 11.8
 //   1 x 4096 -> 4096     9.9 / 18  / 9.4,  5.6      16 x 4096 -> 4096  10.4 / 19 / 9.8, 13.9     128 x 4096 -> 4096  16.5 / 20 / 10.3, 87
 //   256 x 4096 -> 4096  17.4 / 33  / 13.0           512 x 4096 -> 4096 17.5 / 34 / 19.4          784 x 1024 -> 1024  7.7 / 9.8 / 9.2
@@ -442,7 +442,7 @@ static FewTiles few_tiles_form(const Context &c, const ConvProblem &p)
   }
   // estimates in ns, fitted to the figures above
   const double split = igemm_split_estimate(c, p);
-  const double persistent = few ? 1e30 : 2700 + p.Cin * 384 / 95.0;
+  const double persistent = few ? 1e30 : 3000 + p.Cin * 384 / 108.0;
   const double best = split >= 0 && split < persistent ? split : persistent;
   if (!(c.opt_tune & 16) && gemm_fewrows_supported(p)) {
     // a round: each of a CTA's eight warps takes a row, 512 bytes of it at a time; an SM's CTAs overlap only partly
@@ -460,7 +460,8 @@ static FewTiles few_tiles_form(const Context &c, const ConvProblem &p)
 // 14x14x256 -> 77: 20.6 / 21.6). Spatial kernels on channel slabs of 32 bytes, up to 192 output channels: 56x56x96 -> 96
 // at batch 32 43.9 / 27.4, 28x28x160 -> 160 24.9 / 18.8, 56x56x32 -> 64 at batch 64 29.5 / 22.6, 28x28x32 -> 128 11.7 /
 // 11.8; 32 -> 256 13.3 / 16.9, 224 -> 224 18.4 / 19.4. Slabs of 64 bytes, up to 64 channels and enough tiles: 56x56x64
-// -> 64 at batch 64 36.4 / 30.8, at batch 16 13.0 / 12.5; one image 5.3 / 6.7.
+// -> 64 at batch 64 36.4 / 30.8, at batch 16 13.0 / 12.5; one image 5.3 / 6.7. (The spatial kernels whose weights fit an
+// SM do not come here: conv_halo_tc.cu takes them first.)
 static bool gather_first(const Context &c, const ConvProblem &p)
 {
   if (c.opt_split_k != 0 || !conv_gather_tc_supported(p)) return false;
@@ -473,8 +474,14 @@ static bool gather_first(const Context &c, const ConvProblem &p)
 
 bool launch_conv(Context &c, const ConvProblem &p)
 {
-  if (!c.opt_force_generic && c.opt_split_k == 0 && !(c.opt_tune & 64) && conv_halo_tc_supported(c, p)) return launch_conv_halo_tc(c, p);
-  switch (few_tiles_form(c, p)) {
+  const FewTiles few = few_tiles_form(c, p);
+  if (!c.opt_force_generic && c.opt_split_k == 0) {
+    // a spatial kernel whose weights fit an SM: conv_halo_tc.cu, unless so few tiles share so long a reduction that a
+    // cluster is faster (3x3 7x7x512 -> 512, one image: 9.9 us against 7.1; 14x14x256 -> 256 6.1 against 6.4)
+    const double halo = conv_halo_tc_estimate(c, p);
+    if (halo >= 0 && !(few == FewTiles::split && igemm_split_estimate(c, p) < halo)) return launch_conv_halo_tc(c, p);
+  }
+  switch (few) {
     case FewTiles::rows: return launch_gemm_fewrows(c, p);
     case FewTiles::gather: return launch_conv_gather_tc(c, p);
     case FewTiles::split: return launch_igemm_split(c, p);

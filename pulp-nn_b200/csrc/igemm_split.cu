@@ -12,7 +12,8 @@
 // What bounds it: the fixed cost of a kernel (launch, barriers, tensor memory, one round trip to L2, the exchange:
 // some 4 us), then the bytes into an SM. Columns and slices are chosen by plan_split's estimate of both. Measured (us,
 // graph replay; the two-kernel split through scratch or dp4a before): 4096 -> 4096 at 128 vectors 87 -> 10.3, at 256
-// 17.4 -> 12.5 (50 MB into the SMs), 14x14x512 -> 512 of one image 13.7 -> 4.6, 7x7x1024 -> 1024 at batch 4 19.8 -> 5.7.
+// 17.4 -> 12.5 (50 MB into the SMs), 14x14x512 -> 512 of one image 13.7 -> 4.1 (5.6 with the tile
+// put together in shared memory, which a tile of one CTA does without), 7x7x1024 -> 1024 at batch 4 19.8 -> 5.7.
 #include "internal.cuh"
 #include "split_epilogue.cuh"
 #include "sm100_primitives.cuh"
@@ -34,6 +35,7 @@ struct SplitParams {
   int m_tiles, n_tiles, bn;
   int k_split, slabs_per, slabs;
   int stages, tmem_cols;
+  int direct;              // one CTA per tile and whole 16-byte pieces: rows leave from registers
   int const_weights;       // W belongs to a network: no kernel writes it
   int conv, tw_log2, tiles_x, tiles_y, chunks_per_tap, kx, sx, sy, pl, pt, Ho, Wo;    // as in igemm_tc.cu
   int *status;
@@ -142,11 +144,31 @@ igemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   dead = __syncthreads_or(dead);
   tc_fence_after();
   const int m0 = mt * SBM;
-  split_epilogue<MODE>(g.epi, g.out, g.N, g.bn, g.k_split, ks, n0, ncols, ring, tmem, par_k, par_l, dead, [&](int r) -> long long {
+  auto row_of = [&](int r) -> long long {
     if (!g.conv) return m0 + r < g.M ? m0 + r : -1;
     const int y = cy + (r >> g.tw_log2), x = cx + (r & ((1 << g.tw_log2) - 1));
     return y < g.Ho && x < g.Wo ? ((long long)cb * g.Ho + y) * g.Wo + x : -1;
-  });
+  };
+  if (MODE != EPI_RAW32 && g.direct) {
+    if (!dead) {
+      const int quad = warp & 3;
+      const long long row = row_of(quad * 32 + (tid & 31));
+      uint8_t *out = static_cast<uint8_t *>(g.out) + (size_t)(row < 0 ? 0 : row) * g.N + n0;
+      for (int c0 = (warp >> 2) * 32; c0 < ncols; c0 += 64) {
+        uint32_t v[32];
+        tmem_ld_32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
+        tmem_wait_ld();
+        unsigned w[8];
+        requant32_cols<MODE == EPI_RAW32 ? EPI_NONE : MODE>(v, c0, ncols, par_k, par_l, g.epi, g.K, w);
+        if (row >= 0) {
+          *reinterpret_cast<uint4 *>(out + c0) = make_uint4(w[0], w[1], w[2], w[3]);
+          if (c0 + 16 < ncols) *reinterpret_cast<uint4 *>(out + c0 + 16) = make_uint4(w[4], w[5], w[6], w[7]);
+        }
+      }
+    }
+  } else {
+    split_epilogue<MODE>(g.epi, g.out, g.N, g.bn, g.k_split, ks, n0, ncols, ring, tmem, par_k, par_l, dead, row_of);
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -221,6 +243,7 @@ double plan_split(const ConvProblem &p, int sms, SplitParams &g, int &bkb, int &
   if (m_tiles > 2 * sms) return -1;
   g.m_tiles = (int)m_tiles;
   g.slabs = (g.K + bkb - 1) / bkb;
+  const bool pieces = p.epi.mode != EPI_RAW32 && p.Cout % 16 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
   double best = -1;
   bool best_two = false;
   for (int bn = 256; bn >= 32; bn /= 2) {
@@ -238,12 +261,14 @@ double plan_split(const ConvProblem &p, int sms, SplitParams &g, int &bkb, int &
       const double l2 = (double)g.m_tiles * nt * g.slabs * bkb * (SBM + bn) / 9000.0;
       const double mma = (two ? 2.0 : 1.0) * per * bkb / 32 * bn / 3.8;
       double t = load > l2 ? load : l2;
-      t = (t > mma ? t : mma) + bn * 6.0 + 25.0 * bn / split + (split > 1 ? 400.0 + 512.0 * bn * (split - 1) / split / 40.0 : 0.0);
+      t = (t > mma ? t : mma) + bn * 6.0 + (split == 1 && pieces ? 0.0 : 25.0 * bn / split) +
+          (split > 1 ? 400.0 + 512.0 * bn * (split - 1) / split / 40.0 : 0.0);
       if (best < 0 || t < best) { best = t; best_two = two; g.bn = bn; g.n_tiles = nt; g.k_split = split; g.slabs_per = per; }
     }
   }
   if (best < 0) return -1;
   g.tmem_cols = g.bn;
+  g.direct = pieces && g.k_split == 1;
   const int stage = (SBM + g.bn) * bkb, tile = SBM * (g.bn + 4) * 4;
   int stages = ((best_two || g.slabs_per * stage <= SPLIT_SMEM_TWO ? SPLIT_SMEM_TWO : SPLIT_SMEM) - 1024) / stage;
   if (stages > MAX_S_STAGES) stages = MAX_S_STAGES;

@@ -267,8 +267,8 @@ class Stager {
 // ---------------------------------------------------------------------------------------------
 bool launch_conv(Context &c, const ConvProblem &p);             // picks tensor-core or generic
 bool launch_conv_generic(Context &c, const ConvProblem &p);
-// stride-1 spatial kernels with every input pixel fetched once per tile
-bool conv_halo_tc_supported(const Context &c, const ConvProblem &p);
+// spatial kernels with every input pixel fetched once per tile (estimated ns, -1 where that kernel does not take it)
+double conv_halo_tc_estimate(const Context &c, const ConvProblem &p);
 bool launch_conv_halo_tc(Context &c, const ConvProblem &p);
 // any channel count and alignment on the tensor cores, the im2col rows gathered by the warps
 bool conv_gather_tc_supported(const ConvProblem &p);

@@ -33,6 +33,39 @@ __device__ __forceinline__ void stage_channel_params(const Epilogue &e, int n0, 
   }
 }
 
+// 32 accumulator columns c0.. of the calling lane's row -> 32 bytes, parameters staged by stage_channel_params (whole
+// warps: 64-bit parameters are looked at together). Columns past ncols give bytes nobody may store.
+template <int MODE>
+__device__ __forceinline__ void requant32_cols(const uint32_t (&v)[32], int c0, int ncols, const long long *par_k, const long long *par_l,
+                                               const Epilogue &e, int K, unsigned (&w)[8])
+{
+  const int lane = threadIdx.x & 31;
+  const bool fits = MODE == EPI_BN64 &&
+      __all_sync(0xffffffffu, c0 + lane >= ncols || bn_fits_32(par_k[c0 + lane], par_l[c0 + lane], acc_bound(K), e.shift));
+#pragma unroll
+  for (int j = 0; j < 32; j += 4) {
+    int t[4];
+    // columns past the last channel read stale parameters; their bytes are never stored
+    if (MODE == EPI_BN32) {
+      const int4 kk = *reinterpret_cast<const int4 *>(reinterpret_cast<const int *>(par_k) + c0 + j);
+      const int4 ll = *reinterpret_cast<const int4 *>(reinterpret_cast<const int *>(par_l) + c0 + j);
+      t[0] = (int)((unsigned)kk.x * v[j] + (unsigned)ll.x) >> e.shift;
+      t[1] = (int)((unsigned)kk.y * v[j + 1] + (unsigned)ll.y) >> e.shift;
+      t[2] = (int)((unsigned)kk.z * v[j + 2] + (unsigned)ll.z) >> e.shift;
+      t[3] = (int)((unsigned)kk.w * v[j + 3] + (unsigned)ll.w) >> e.shift;
+    } else if (MODE == EPI_BN64) {
+      requant4_bn64(par_k + c0 + j, par_l + c0 + j, v[j], v[j + 1], v[j + 2], v[j + 3], e.shift, fits, t);
+    } else {
+      const int4 bb = *reinterpret_cast<const int4 *>(reinterpret_cast<const int *>(par_l) + c0 + j);
+      const int a4[4] = {(int)v[j] + bb.x, (int)v[j + 1] + bb.y, (int)v[j + 2] + bb.z, (int)v[j + 3] + bb.w};
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        t[u] = MODE == EPI_MULT ? (int)(short)((int)((unsigned)e.out_mult * (unsigned)a4[u]) >> e.shift) : a4[u] >> e.shift;
+    }
+    w[j >> 2] = pack4_sat_u8(t[0], t[1], t[2], t[3]);
+  }
+}
+
 template <int MODE>
 __device__ __forceinline__ int requant_param(int a, int col, const long long *par_k, const long long *par_l, const Epilogue &e)
 {

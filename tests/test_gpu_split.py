@@ -53,3 +53,14 @@ def test_convolution(H, W, Cin, Cout, k, s, p, batch, gpu, restatement):
     c = wl.conv_case(94, H, W, Cin, Cout, kernel=(k, k), strides=(s, s), pads=(p, p, p, p), batch=batch, out_shift=13)
     same(gpu.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)),
          restatement.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
+
+
+# one CTA per tile, whole 16-byte pieces: the rows leave from registers. The last tile's columns end at half a piece of 32.
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("relu,bn", MODES)
+@pytest.mark.parametrize("M,K,N", [(196, 512, 512), (131, 528, 304), (49, 512, 1040)])
+def test_rows_from_registers(M, K, N, bits, relu, bn, gpu, restatement):
+    c = wl.pointwise_case(95, 1, M, K, N, bits=bits, out_shift=11, with_bias=True, out_mult=3, relu=relu, bn=bn,
+                          k_range=(-64, 64), lam_range=(-2 ** 20, 2 ** 20))
+    same(gpu.pointwise(bits, c["x"], c["w"], c["k"], c["lam"], **pw_kw(c)),
+         restatement.pointwise(bits, c["x"], c["w"], c["k"], c["lam"], **pw_kw(c)))
