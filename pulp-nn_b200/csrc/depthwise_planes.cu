@@ -25,6 +25,7 @@ namespace pulpnn {
 namespace {
 
 constexpr int DT = 256;
+constexpr int PLANES_SMEM = 200 * 1024;      // planes and expanded filter rows of a CTA
 
 struct PlanesParams {
   DepthwiseProblem p;
@@ -275,7 +276,7 @@ bool launch_planes(Context &c, const PlanesParams &g, int smem)
   auto kern = depthwise_planes_kernel<MODE, K, S, CG>;
   static PerDeviceInt attr_set;
   if (!attr_set.get(c.device)) {
-    if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), "cudaFuncSetAttribute(depthwise_planes)"))
+    if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PLANES_SMEM), "cudaFuncSetAttribute(depthwise_planes)"))
       return false;
     attr_set.set(c.device, 1);
   }
@@ -297,7 +298,8 @@ bool launch_planes_mode(Context &c, const PlanesParams &g, int cg, int smem)
   return cg == 16 ? launch_planes_ks<MODE, 16>(c, g, smem) : launch_planes_ks<MODE, 32>(c, g, smem);
 }
 
-// lays the work out; false when not even one band of R rows fits shared memory or the grid is too large
+// lays the work out; false when not even one band of R rows and the filter rows fit shared memory or the grid is too
+// large
 bool configure(const DepthwiseProblem &p, int sms, PlanesParams &g, int &cg, int &smem)
 {
   const int S = p.sx, K = p.kx, R = S == 1 ? 4 : 2;
@@ -318,7 +320,8 @@ bool configure(const DepthwiseProblem &p, int sms, PlanesParams &g, int &cg, int
   while (blocks > 1 && (plane_of(blocks * R) * cg > 48 * 1024 || (long long)p.B * g.groups * ((rb + blocks - 1) / blocks) < 2LL * sms))
     blocks = (blocks + 1) / 2;
   g.band = blocks * R;
-  if (plane_of(g.band) * cg > 200 * 1024) return false;
+  const int filters = K * (4 / S) * 2 * cg * 4;
+  if (plane_of(g.band) * cg + filters > PLANES_SMEM) return false;
   // 32-bit offsets inside a group of channels, the rows above and below its image included
   if (((long long)cg * p.H + p.pt + g.band * S + K) * p.W > 0x7fff0000LL) return false;
   if ((long long)p.Ho * p.Wo * p.C > 0x7fff0000LL || ((long long)p.H + p.pt + g.band * S + K) * p.W * p.C > 0x7fff0000LL) return false;
@@ -327,7 +330,7 @@ bool configure(const DepthwiseProblem &p, int sms, PlanesParams &g, int &cg, int
   g.row_pitch = (int)pitch;
   g.rows_in = (g.band - 1) * S + K;
   g.plane = (int)plane_of(g.band);
-  smem = g.plane * cg + K * (4 / S) * 2 * cg * 4;
+  smem = g.plane * cg + filters;
   g.by_groups.set((unsigned)g.groups);
   g.by_bands.set((unsigned)g.bands);
   const int piece = p.in_is_hwc ? 4 : 16;

@@ -40,6 +40,22 @@ def test_shapes(k, s, hwc, H, W, C, batch, gpu, restatement):
          restatement.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
 
 
+# the widest rows whose band and filter rows fit a CTA's shared memory, the first that do not, and the last whose band
+# alone would: each is followed by an ordinary call, which has to find nothing left over
+@pytest.mark.parametrize("k,s,hwc,H,W,C", [
+    (5, 1, True, 8, 772, 20), (5, 1, True, 8, 773, 20), (5, 1, True, 8, 784, 40), (5, 1, True, 8, 792, 20), (5, 1, True, 8, 793, 20),
+    (5, 1, False, 8, 764, 20), (5, 1, False, 8, 776, 20), (5, 1, False, 8, 780, 20), (5, 2, True, 6, 896, 20), (5, 2, True, 6, 900, 20),
+    (5, 2, False, 6, 888, 20), (5, 2, False, 6, 904, 20), (5, 1, True, 5, 1580, 8), (3, 1, True, 4, 1044, 30), (3, 1, True, 4, 1050, 30),
+    (3, 1, True, 4, 1048, 64), (3, 1, True, 4, 1060, 30), (3, 1, False, 4, 1036, 20), (3, 1, False, 4, 1044, 20), (3, 1, False, 4, 1052, 20),
+    (3, 2, True, 6, 1264, 30), (3, 2, True, 6, 1270, 30), (3, 1, True, 4, 2120, 7)])
+def test_widest_rows(k, s, hwc, H, W, C, gpu, restatement):
+    p = k // 2
+    for h, w, c in ((H, W, C), (9, 7, 20)):
+        c = wl.depthwise_case(83, h, w, c, kernel=(k, k), strides=(s, s), pads=(p, p, p, p), out_shift=9, hwc=hwc)
+        same(gpu.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)),
+             restatement.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
+
+
 @pytest.mark.parametrize("hwc", [False, True])
 @pytest.mark.parametrize("shift", [1, 2, 3])
 def test_unaligned_input(hwc, shift, gpu, restatement):
