@@ -284,7 +284,8 @@ double plan_halo(const ConvProblem &p, int sms, HaloParams &g, int &bkb, int &sm
   double best = -1;
   for (int nt = (p.Cout + 255) / 256;; nt++) {
     const int bn = ((p.Cout + nt - 1) / nt + 15) & ~15, n_tiles = (p.Cout + bn - 1) / bn;
-    if (nt > (p.Cout + 255) / 256 && (bn < 32 || n_tiles > sms)) break;
+    // (with more channel tiles than SMs not even the first candidate has a round)
+    if (n_tiles > sms || (nt > (p.Cout + 255) / 256 && bn < 32)) break;
     const long long fixed = (long long)g.K * bn + 1024;
     const long long boxes = (HALO_SMEM - fixed) / g.box_stride;
     if (fixed >= HALO_SMEM || boxes < 2) continue;

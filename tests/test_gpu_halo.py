@@ -52,3 +52,11 @@ def test_shapes(H, W, Cin, Cout, kernel, pads, batch, strides, gpu, restatement)
     x = c["x"]
     for b in (0, batch // 2, batch - 1):
         same(got[b:b + 1], restatement.conv(32, x[b:b + 1], c["w"], c["k"], c["lam"], **conv_kw(c)))
+
+
+# the most channels whose tiles find an SM each on 148 SMs, and more tiles than SMs, which are for other kernels
+@pytest.mark.parametrize("Cin,Cout,kernel", [(32, 37888, (3, 3)), (32, 37904, (3, 3)), (64, 40000, (1, 3)), (32, 65520, (3, 1))])
+def test_more_channel_tiles_than_sms(Cin, Cout, kernel, gpu, restatement):
+    c = wl.conv_case(112, 4, 4, Cin, Cout, kernel=kernel, pads=(kernel[0] // 2,) * 2 + (kernel[1] // 2,) * 2, out_shift=12)
+    same(gpu.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)),
+         restatement.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
