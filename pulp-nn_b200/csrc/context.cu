@@ -43,9 +43,12 @@ void set_error(int code, const char *fmt, ...)
   va_end(ap);
 }
 
+// Records a failure, and takes it from the runtime too: the runtime keeps the code of a failed call for the next
+// cudaGetLastError(), where a later call would report it as its own.
 bool cuda_ok(cudaError_t e, const char *what)
 {
   if (e == cudaSuccess) return true;
+  cudaGetLastError();
   set_error(PULPNN_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   return false;
 }

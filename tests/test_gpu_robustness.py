@@ -98,3 +98,19 @@ def test_second_device_in_the_same_process(restatement):
             assert api.device_status() == 0
     finally:
         pulpnn.GpuKernels(device=0)
+
+
+def test_a_failed_call_leaves_nothing_for_the_next(restatement):
+    """A call that CUDA refuses (host buffers of 2^31 images, for which no staging buffer can be had) raises, and the
+    ordinary call after it does not."""
+    gpu = pulpnn.GpuKernels()
+    x = np.zeros((1, 4, 4, 16), np.uint8)
+    api.set_batch(2 ** 31 - 1)
+    try:
+        with pytest.raises(pulpnn.PulpNNError):
+            api.pulp_nn_maxpool(32, x, x, 1000, 1000, 64, 1000, 1000, 1, 1, 0, 0, 0, 0, 1, 1)
+    finally:
+        api.set_batch(1)
+    c = wl.pointwise_case(53, 9, 9, 64, 96, out_shift=9)
+    want = restatement.pointwise(32, c["x"], c["w"], c["k"], c["lam"], out_shift=9)
+    assert np.array_equal(gpu.pointwise(32, c["x"], c["w"], c["k"], c["lam"], out_shift=9), want)
