@@ -88,11 +88,12 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
   // ---- stage the planes -----------------------------------------------------------------------
   if (p.in_is_hwc) {
     constexpr int CQ = CG / 4;
-    // 32-bit offsets into the image from the word at or below its first byte; the words that lie inside the tensor
-    const size_t off = (size_t)b * p.H * p.W * p.C;
+    // 32-bit offsets into the image from the word at or below its first byte
+    const int own = p.H * p.W * p.C;
+    const size_t off = (size_t)b * own;
     const int lead = (int)(reinterpret_cast<uintptr_t>(p.in + off) & 3);
     const uint8_t *img = p.in + off - lead;
-    const int lo = b > 0 ? -64 : lead, hi = lead + p.H * p.W * p.C + (b < p.B - 1 ? 64 : 0);
+    const ImageSpan span(lead, own, off, (size_t)(p.B - 1 - b) * own);
     const int items = g.rows_in * qw;                       // words of four pixels, the thread's four channels
     const int cq = tid % CQ, left = nch - 4 * cq;           // channels of this word that exist
     constexpr int STEP = DT / CQ;
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
         if (g.words) {
 #pragma unroll
           for (int i = 0; i < 4; i++) v[u][i] = ldg4_if(img + at[u] + i * p.C, ok && (unsigned)(ix + i) < (unsigned)p.W);
-        } else if (!ok || ((at[u] & ~3) >= lo && at[u] + 3 * p.C + 8 <= hi)) {
+        } else if (!ok || span.holds_words(at[u], p.C)) {
 #pragma unroll
           for (int i = 0; i < 4; i++) {
             const bool in = ok && (unsigned)(ix + i) < (unsigned)p.W;

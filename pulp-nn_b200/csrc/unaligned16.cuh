@@ -95,6 +95,16 @@ struct Chunk {
   }
 };
 
+// One image of a tensor of bytes, by offsets from the word at or below its first byte (`lead` bytes before it): between
+// lo and hi lie the image's own bytes and up to 64 of the `before` and `after` that the tensor has on either side.
+struct ImageSpan {
+  int lo, hi;
+  __host__ __device__ ImageSpan(int lead, int own, size_t before, size_t after)
+      : lo(lead - (int)(before < 64 ? before : 64)), hi(lead + own + (int)(after < 64 ? after : 64)) {}
+  // four pixels of C bytes from offset `at` on, each read as the two words that its first four bytes lie across
+  __host__ __device__ bool holds_words(int at, int C) const { return (at & ~3) >= lo && at + 3 * C + 8 <= hi; }
+};
+
 // bytes [from, to) of word i of a 16-byte chunk
 __device__ __forceinline__ unsigned word_mask(int i, int from, int to)
 {

@@ -57,6 +57,15 @@ def test_widest_rows(k, s, hwc, H, W, C, gpu, restatement):
 
 
 @pytest.mark.parametrize("hwc", [False, True])
+@pytest.mark.parametrize("H,W,C,batch", [(1, 3, 1, 2), (1, 3, 1, 5), (1, 3, 2, 3), (1, 4, 1, 5), (2, 3, 1, 3), (1, 3, 7, 2), (3, 5, 5, 4)])
+@pytest.mark.parametrize("pr", [0, 1])
+def test_images_of_a_few_bytes(hwc, H, W, C, batch, pr, gpu, restatement):
+    c = wl.depthwise_case(84, H, W, C, batch=batch, pads=(1, 1, 1, pr), out_shift=9, hwc=hwc)
+    same(gpu.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)),
+         restatement.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
+
+
+@pytest.mark.parametrize("hwc", [False, True])
 @pytest.mark.parametrize("shift", [1, 2, 3])
 def test_unaligned_input(hwc, shift, gpu, restatement):
     import torch
