@@ -61,6 +61,9 @@ const char *pulpnn_last_error_message(void);
 void pulpnn_clear_error(void);
 /* kernels launched by this library since it was loaded (all threads) */
 unsigned long long pulpnn_launch_count(void);
+/* The kernel family of the calling thread's latest launch ("igemm_tc_kernel", ...), "" before the first:
+ * which of the kernels that serve an entry point a call took, for tests and measurements. */
+const char *pulpnn_last_kernel(void);
 /* Reads and clears the device-side status word: 0 = every bounded wait in the
  * tensor-core kernels completed. Synchronises the stream first. */
 int  pulpnn_device_status(void);

@@ -125,6 +125,7 @@ def load_library():
     _lib = C.CDLL(MAIN_SO, mode=C.RTLD_GLOBAL)
     _lib.pulpnn_last_error_message.restype = C.c_char_p
     _lib.pulpnn_launch_count.restype = C.c_ulonglong
+    _lib.pulpnn_last_kernel.restype = C.c_char_p
     _lib.pulpnn_net_create.restype = C.c_void_p
     _lib.pulpnn_net_layer_output_bytes.restype = C.c_size_t
     _lib.pulpnn_net_launches_per_run.restype = C.c_ulonglong

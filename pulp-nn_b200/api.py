@@ -90,6 +90,11 @@ def launch_count():
     return int(_lib.load_library().pulpnn_launch_count())
 
 
+def last_kernel():
+    """Kernel family of this thread's latest launch."""
+    return _lib.load_library().pulpnn_last_kernel().decode()
+
+
 def device_status():
     return _lib.load_library().pulpnn_device_status()
 

@@ -233,6 +233,7 @@ int pulpnn_last_error(void) { return ctx().err; }
 const char *pulpnn_last_error_message(void) { return ctx().msg; }
 void pulpnn_clear_error(void) { ctx().err = PULPNN_OK; ctx().msg[0] = 0; }
 unsigned long long pulpnn_launch_count(void) { return g_launches.load(); }
+const char *pulpnn_last_kernel(void) { return thread_last_kernel(); }
 
 int pulpnn_device_status(void)
 {

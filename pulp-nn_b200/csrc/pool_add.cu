@@ -473,7 +473,7 @@ bool launch_maxpool(Context &c, const PoolProblem &p, uint8_t *clobber_in)
     const unsigned blocks = (unsigned)((total + 255) / 256);
     if (vec) maxpool_kernel<true><<<blocks, 256, 0, c.stream>>>(p, CW, total);
     else     maxpool_kernel<false><<<blocks, 256, 0, c.stream>>>(p, CW, total);
-    count_launch();
+    count_launch("maxpool_kernel");
     if (!cuda_ok(cudaGetLastError(), "maxpool launch")) return false;
   } else if (!launch_pool<false>(c, p)) return false;
   if (clobber_in) {
@@ -523,7 +523,7 @@ bool launch_avgpool(Context &c, const PoolProblem &p)
   const unsigned blocks = (unsigned)((total + 255) / 256);
   if (vec) avgpool_kernel<true><<<blocks, 256, 0, c.stream>>>(p, CW, total);
   else     avgpool_kernel<false><<<blocks, 256, 0, c.stream>>>(p, CW, total);
-  count_launch();
+  count_launch("avgpool_kernel");
   return cuda_ok(cudaGetLastError(), "avgpool launch");
 }
 
