@@ -185,6 +185,11 @@ __global__ void __launch_bounds__(256, 2) conv_smallcin_kernel(const SmallParams
 
 }  // namespace
 
+// left padding in whole words; a staged row; weights and parameters of a CTA
+static int staged_lead(const ConvProblem &p) { return (p.pl * p.Cin + 3) & ~3; }
+static int staged_pitch(const ConvProblem &p) { return (staged_lead(p) + (p.W + p.kx) * p.Cin + 16 + 3) & ~3; }
+static size_t fixed_bytes(const ConvProblem &p) { return (size_t)p.ky * RW * CO * 4 + CO * (8 + 8 + 4); }
+
 bool conv_smallcin_supported(const ConvProblem &p)
 {
   if (p.epi.mode == EPI_RAW32) return false;
@@ -192,7 +197,8 @@ bool conv_smallcin_supported(const ConvProblem &p)
   if ((long long)p.W * p.Cin > 16384 || p.B > 65535) return false;
   // the last pixel's three words must end inside a staged row (pitch = lead + (W+kx)*Cin + 16)
   if ((p.Wo - 1) * p.sx - p.pl > p.W + p.kx) return false;
-  return true;
+  // the input rows of one output row fit shared memory
+  return fixed_bytes(p) + (size_t)p.ky * staged_pitch(p) <= 48 * 1024;
 }
 
 bool launch_conv_smallcin(Context &c, const ConvProblem &p)
@@ -200,12 +206,12 @@ bool launch_conv_smallcin(Context &c, const ConvProblem &p)
   SmallParams g;
   g.p = p;
   g.row_bytes = p.W * p.Cin;
-  g.lead = (p.pl * p.Cin + 3) & ~3;
-  g.pitch = (g.lead + (p.W + p.kx) * p.Cin + 16 + 3) & ~3;
+  g.lead = staged_lead(p);
+  g.pitch = staged_pitch(p);
   g.vec_rows = (g.row_bytes % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.in) & 3) == 0);
   g.vec_store = (p.Cout % 16 == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
   if (p.Cout == CO && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0) g.vec_store = 2;
-  const size_t fixed = (size_t)p.ky * RW * CO * 4 + CO * (8 + 8 + 4);
+  const size_t fixed = fixed_bytes(p);
   // strip height: shared memory under 48 KB, and a pixel-pair count close to a multiple of 256
   int best = 1; double best_waste = 1e9;
   for (int ro = 1; ro <= p.Ho && ro <= 64; ro++) {
@@ -219,7 +225,6 @@ bool launch_conv_smallcin(Context &c, const ConvProblem &p)
   g.rows_out = best;
   g.rows_in = (best - 1) * p.sy + p.ky;
   const size_t smem = fixed + (size_t)g.rows_in * g.pitch;
-  if (smem > 48 * 1024) { set_error(PULPNN_ERR_UNSUPPORTED, "conv: one input row strip does not fit in shared memory"); return false; }
   dim3 grid((unsigned)((p.Ho + best - 1) / best), (unsigned)p.B);
   switch (p.epi.mode) {
     case EPI_NONE: conv_smallcin_kernel<EPI_NONE><<<grid, 256, smem, c.stream>>>(g); break;

@@ -504,6 +504,8 @@ bool launch_conv(Context &c, const ConvProblem &p)
   // 56x56x181 -> 250 at batch 8 55 against 719, a 1001 -> 1000 linear layer 6.6 against 52, and 3.8 against 7.3 for the
   // smallest (7x7x16 -> 16, one image). What is left to the dp4a kernel are tensors beyond 32-bit offsets.
   if (!c.opt_force_generic && conv_gather_tc_supported(p)) return launch_conv_gather_tc(c, p);
+  // (first layers among those have a kernel of their own, whatever the batch)
+  if (!c.opt_force_generic && conv_smallcin_supported(p)) return launch_conv_smallcin(c, p);
   return launch_conv_generic(c, p);
 }
 
