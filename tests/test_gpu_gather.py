@@ -11,6 +11,7 @@ from test_gpu_parity import MODES, conv_kw, pw_kw, same
 
 pytestmark = pytest.mark.gpu
 api, wl = pulpnn.api, pulpnn.workloads
+KERNEL = "conv_gather_tc_kernel"
 
 
 @pytest.fixture(scope="module")
@@ -29,8 +30,9 @@ def _status():
 def test_modes(bits, relu, bn, gpu, restatement):
     c = wl.conv_case(70, 13, 11, 21, 37, strides=(1, 2), batch=3, bits=bits, out_shift=9, with_bias=True, out_mult=3,
                      relu=relu, bn=bn, w_range=(-128, 127), k_range=(-64, 64), lam_range=(-2 ** 20, 2 ** 20))
-    same(gpu.conv(bits, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)),
-         restatement.conv(bits, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
+    got = gpu.conv(bits, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c))
+    assert api.last_kernel() == KERNEL
+    same(got, restatement.conv(bits, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
 
 
 CONVS = [  # H, W, Cin, Cout, kernel, strides, pads (top, bottom, left, right), batch
@@ -50,19 +52,22 @@ CONVS = [  # H, W, Cin, Cout, kernel, strides, pads (top, bottom, left, right), 
 def test_convolutions(H, W, Cin, Cout, kernel, strides, pads, batch, gpu, restatement):
     c = wl.conv_case(71, H, W, Cin, Cout, kernel=kernel, strides=strides, pads=pads, batch=batch, out_shift=10,
                      with_bias=True, w_range=(-128, 127))
-    same(gpu.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)),
-         restatement.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
+    got = gpu.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c))
+    assert api.last_kernel() == KERNEL
+    same(got, restatement.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
 
 
 @pytest.mark.parametrize("cin,cout", [(1, 1), (15, 16), (17, 20), (31, 3), (127, 130), (129, 64), (257, 256), (1000, 999), (4095, 70)])
 def test_pointwise_and_linear(cin, cout, gpu, restatement):
     c = wl.pointwise_case(72, 9, 15, cin, cout, batch=2, out_shift=9, with_bias=True, w_range=(-128, 127))
-    same(gpu.pointwise(32, c["x"], c["w"], c["k"], c["lam"], **pw_kw(c)),
-         restatement.pointwise(32, c["x"], c["w"], c["k"], c["lam"], **pw_kw(c)))
+    got = gpu.pointwise(32, c["x"], c["w"], c["k"], c["lam"], **pw_kw(c))
+    assert api.last_kernel() == KERNEL
+    same(got, restatement.pointwise(32, c["x"], c["w"], c["k"], c["lam"], **pw_kw(c)))
     for batch in (1, 130):
         c = wl.linear_case(73, cin, cout, batch=batch, with_bias=True)
-        same(gpu.linear_out_32(c["x"], c["w"], bias32=c["bias32"]),
-             restatement.linear_out_32(c["x"], c["w"], bias32=c["bias32"]))
+        got = gpu.linear_out_32(c["x"], c["w"], bias32=c["bias32"])
+        assert api.last_kernel() == KERNEL
+        same(got, restatement.linear_out_32(c["x"], c["w"], bias32=c["bias32"]))
 
 
 @pytest.mark.parametrize("shift_in,shift_w,shift_out", [(1, 0, 0), (0, 3, 0), (8, 8, 4), (5, 2, 1)])
@@ -79,6 +84,7 @@ def test_unaligned_buffers(shift_in, shift_w, shift_out, gpu, restatement):
     api.pulp_nn_conv_Ho_parallel(32, x[shift_in:], None, None, out[shift_out:], w[shift_w:], k, lam, 1, 12, 10, 9, 32,
                                  10, 9, 48, 3, 3, 1, 1, 1, 1, 1, 1, 1, 1)
     api.synchronize()
+    assert api.last_kernel() == KERNEL
     got = out.cpu().numpy()
     same(got[shift_out:shift_out + want.size].reshape(want.shape), want)
     assert (got[:shift_out] == 0xA5).all() and (got[shift_out + want.size:] == 0xA5).all()

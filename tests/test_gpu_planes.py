@@ -9,6 +9,7 @@ from test_gpu_parity import MODES, dw_kw, same
 
 pytestmark = pytest.mark.gpu
 api, wl = pulpnn.api, pulpnn.workloads
+KERNEL = "depthwise_planes_kernel"
 
 
 @pytest.fixture(scope="module")
@@ -23,8 +24,9 @@ def test_modes(bits, relu, bn, hwc, gpu, restatement):
     c = wl.depthwise_case(80, 13, 11, 37, kernel=(5, 5), pads=(2, 2, 2, 2), batch=2, bits=bits, out_shift=8,
                           with_bias=True, out_mult=3, relu=relu, bn=bn, w_range=(-128, 127), k_range=(-64, 64),
                           lam_range=(-2 ** 20, 2 ** 20), hwc=hwc)
-    same(gpu.depthwise(bits, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)),
-         restatement.depthwise(bits, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
+    got = gpu.depthwise(bits, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c))
+    assert api.last_kernel() == KERNEL
+    same(got, restatement.depthwise(bits, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
 
 
 @pytest.mark.parametrize("k", [3, 5])
@@ -36,24 +38,27 @@ def test_shapes(k, s, hwc, H, W, C, batch, gpu, restatement):
     p = k // 2
     c = wl.depthwise_case(81, H, W, C, kernel=(k, k), strides=(s, s), pads=(p, p, p, p), batch=batch, out_shift=9,
                           with_bias=True, hwc=hwc)
-    same(gpu.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)),
-         restatement.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
+    got = gpu.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c))
+    assert api.last_kernel() == KERNEL
+    same(got, restatement.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
 
 
 # the widest rows whose band and filter rows fit a CTA's shared memory, the first that do not, and the last whose band
 # alone would: each is followed by an ordinary call, which has to find nothing left over
-@pytest.mark.parametrize("k,s,hwc,H,W,C", [
-    (5, 1, True, 8, 772, 20), (5, 1, True, 8, 773, 20), (5, 1, True, 8, 784, 40), (5, 1, True, 8, 792, 20), (5, 1, True, 8, 793, 20),
-    (5, 1, False, 8, 764, 20), (5, 1, False, 8, 776, 20), (5, 1, False, 8, 780, 20), (5, 2, True, 6, 896, 20), (5, 2, True, 6, 900, 20),
-    (5, 2, False, 6, 888, 20), (5, 2, False, 6, 904, 20), (5, 1, True, 5, 1580, 8), (3, 1, True, 4, 1044, 30), (3, 1, True, 4, 1050, 30),
-    (3, 1, True, 4, 1048, 64), (3, 1, True, 4, 1060, 30), (3, 1, False, 4, 1036, 20), (3, 1, False, 4, 1044, 20), (3, 1, False, 4, 1052, 20),
-    (3, 2, True, 6, 1264, 30), (3, 2, True, 6, 1270, 30), (3, 1, True, 4, 2120, 7)])
-def test_widest_rows(k, s, hwc, H, W, C, gpu, restatement):
+@pytest.mark.parametrize("k,s,hwc,H,W,C,fits", [
+    (5, 1, True, 8, 772, 20, 1), (5, 1, True, 8, 773, 20, 0), (5, 1, True, 8, 784, 40, 0), (5, 1, True, 8, 792, 20, 0),
+    (5, 1, True, 8, 793, 20, 0), (5, 1, False, 8, 764, 20, 1), (5, 1, False, 8, 776, 20, 0), (5, 1, False, 8, 780, 20, 0),
+    (5, 2, True, 6, 896, 20, 1), (5, 2, True, 6, 900, 20, 0), (5, 2, False, 6, 888, 20, 1), (5, 2, False, 6, 904, 20, 0),
+    (5, 1, True, 5, 1580, 8, 0), (3, 1, True, 4, 1044, 30, 1), (3, 1, True, 4, 1050, 30, 0), (3, 1, True, 4, 1048, 64, 0),
+    (3, 1, True, 4, 1060, 30, 0), (3, 1, False, 4, 1036, 20, 1), (3, 1, False, 4, 1044, 20, 0), (3, 1, False, 4, 1052, 20, 0),
+    (3, 2, True, 6, 1264, 30, 1), (3, 2, True, 6, 1270, 30, 0), (3, 1, True, 4, 2120, 7, 0)])
+def test_widest_rows(k, s, hwc, H, W, C, fits, gpu, restatement):
     p = k // 2
-    for h, w, c in ((H, W, C), (9, 7, 20)):
+    for h, w, c, planes in ((H, W, C, fits), (9, 7, 20, 1)):
         c = wl.depthwise_case(83, h, w, c, kernel=(k, k), strides=(s, s), pads=(p, p, p, p), out_shift=9, hwc=hwc)
-        same(gpu.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)),
-             restatement.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
+        got = gpu.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c))
+        assert (api.last_kernel() == KERNEL) == bool(planes)
+        same(got, restatement.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
 
 
 @pytest.mark.parametrize("hwc", [False, True])
@@ -61,8 +66,9 @@ def test_widest_rows(k, s, hwc, H, W, C, gpu, restatement):
 @pytest.mark.parametrize("pr", [0, 1])
 def test_images_of_a_few_bytes(hwc, H, W, C, batch, pr, gpu, restatement):
     c = wl.depthwise_case(84, H, W, C, batch=batch, pads=(1, 1, 1, pr), out_shift=9, hwc=hwc)
-    same(gpu.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)),
-         restatement.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
+    got = gpu.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c))
+    assert api.last_kernel() == KERNEL
+    same(got, restatement.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
 
 
 @pytest.mark.parametrize("hwc", [False, True])
@@ -79,6 +85,7 @@ def test_unaligned_input(hwc, shift, gpu, restatement):
     fn(32, x[shift:], None, None, out[shift:], put(c["w"]), None, put(c["k"]), put(c["lam"]), 1, 9, 13, 9, 20, 13, 9, 20,
        5, 5, 2, 2, 2, 2, 1, 1, 1, 1)
     api.synchronize()
+    assert api.last_kernel() == KERNEL
     got = out.cpu().numpy()
     same(got[shift:shift + want.size].reshape(want.shape), want)
     assert (got[:shift] == 0xA5).all() and (got[shift + want.size:] == 0xA5).all()

@@ -38,6 +38,21 @@ def test_windows_that_pads_shift(gpu, restatement):
         same(gpu.avgpool(32, x, **kw), restatement.avgpool(32, x, **kw))
 
 
+@pytest.mark.parametrize("H,W,k,kernel", [(560, 560, (16, 16), "pool_kernel"), (100, 257 * 13, (1, 257), "pool_kernel"),
+                                          (100, 258 * 13, (1, 258), "avgpool_kernel")])
+def test_largest_sums(H, W, k, kernel, gpu, restatement):
+    """Windows of up to 257 pixels are summed in 16 bits: 257 * 255 is 65535. More than 1184 of them at a channel count of
+    no whole words, so that they do not go to the kernel with a block per window."""
+    x = np.full((1, H, W, 21), 255, np.uint8)
+    x[:, : k[0], : k[1]] = np.random.default_rng(8).integers(0, 256, size=(1, k[0], k[1], 21), dtype=np.uint8)
+    kw = dict(out_hw=(H // k[0], W // k[1]), kernel=k, pads=(0, 0, 0, 0), strides=k)
+    for bits, requant in ((32, 0), (32, 1), (64, 1)):
+        q = dict(lam=77, out_shift=6, out_add=-50, requant=requant)
+        got = gpu.avgpool(bits, x, **q, **kw)
+        assert api.last_kernel() == kernel
+        same(got, restatement.avgpool(bits, x, **q, **kw))
+
+
 @pytest.mark.parametrize("shift", [0, 1, 4])
 @pytest.mark.parametrize("shape", [(1, 1, 1, 1), (1, 1, 1, 15), (2, 3, 5, 7), (3, 9, 9, 48), (5, 31, 33, 37)])
 def test_add(shape, shift, gpu, restatement):
