@@ -255,13 +255,13 @@ bool launch_halo_bk(Context &c, const CUtensorMap &a, const CUtensorMap &w, cons
   return launch_halo<MODE, 128>(c, a, w, g, grid, smem);
 }
 
-// Lays the problem out and returns the estimated ns, -1 where it does not fit or igemm_tc.cu is faster. The channels
-// are cut into the tiles with the least estimated time: an MMA takes 80 cycles or BN / 2, whichever is more, a row of a TMA box some 12,
-// the CTA's slice of W 80 bytes per ns, and the tiles come in rounds of as many as there are SMs. Cutting the channels
-// multiplies the MMAs that narrow tiles leave half idle: beyond twice those of one tile, and more than two rounds,
-// igemm_tc.cu is faster (14x14x256 -> 256 at batch 64, four tiles of 64: 17.8 us against 12.9; 28x28x224 -> 224 at
-// batch 16 19.9 / 18.3; 28x28x160 -> 160 at batch 32 18.8 / 19.1; in one or two rounds 14x14x256 at batch 32 10.8 /
-// 12.3, at batch 8 6.6 / 10.4).
+// Lays the problem out and returns the estimated ns, -1 where it does not fit. The channels are cut into the tiles with
+// the least estimated time: an MMA takes 80 cycles or BN / 2, whichever is more, a row of a TMA box some 12, the CTA's
+// slice of W 80 bytes per ns, and the tiles come in rounds of as many as there are SMs. Cutting the channels multiplies
+// the MMAs that narrow tiles leave half idle: beyond twice those of one tile, and more than two rounds, igemm_tc.cu is
+// faster (-1 as well: 14x14x256 -> 256 at batch 64, four tiles of 64: 17.8 us against 12.9; 28x28x224 -> 224 at batch 16
+// 19.9 / 18.3; 28x28x160 -> 160 at batch 32 18.8 / 19.1; in one or two rounds 14x14x256 at batch 32 10.8 / 12.3, at
+// batch 8 6.6 / 10.4).
 double plan_halo(const ConvProblem &p, int sms, HaloParams &g, int &bkb, int &smem)
 {
   if (p.sx < 1 || p.sx > 2 || p.sy < 1 || p.sy > 2 || p.ky * p.kx < 2 || p.kx > 9 || p.ky > 9 || p.Cin % 32 != 0 || p.Cout % 16 != 0)
@@ -305,7 +305,13 @@ double plan_halo(const ConvProblem &p, int sms, HaloParams &g, int &bkb, int &sm
   while (g.acc_cols < g.bn) g.acc_cols *= 2;
   g.n_acc = 512 / g.acc_cols < MAX_ACC ? 512 / g.acc_cols : MAX_ACC;
   g.wide_store = p.Cout % 32 == 0 && g.bn % 32 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
-  return best;
+  // What the cut takes, to be compared with other kernels' estimates: fitted to 188 calls of 3 to 80 us over odd image
+  // sizes, strides and kernels (standard deviation 9 %). The start of a chunk and of a tile cost the MMA thread some 480
+  // and 930 cycles, a row of a box 2.3 to 3.9 in the long run.
+  const double rounds = (double)((m_tiles + sms / g.n_tiles - 1) / (sms / g.n_tiles));
+  const double mma = 0.94 * p.ky * p.kx * (p.Cin / 32) * (g.bn > 160 ? g.bn / 2.0 : 80.0) + 480.0 * g.chunks + 930;
+  const double rows = (bkb == 128 ? 3.9 : (bkb == 64 ? 3.05 : 2.3)) * g.chunks * p.sx * p.sy * g.box_w * g.box_h;
+  return 2470 + rounds * (mma > rows ? mma : rows) / 1.9 + (double)g.K * g.bn / 46;
 }
 
 }  // namespace
@@ -315,7 +321,7 @@ double conv_halo_tc_estimate(const Context &c, const ConvProblem &p)
   HaloParams g = {};
   int bkb, smem;
   const double ns = plan_halo(p, c.sm_count > 0 ? c.sm_count : 148, g, bkb, smem);
-  return ns < 0 || !encode_tiled_fn() ? -1 : 2000 + ns;
+  return encode_tiled_fn() ? ns : -1;
 }
 
 bool launch_conv_halo_tc(Context &c, const ConvProblem &p)

@@ -286,7 +286,10 @@ double igemm_split_estimate(const Context &c, const ConvProblem &p)
   SplitParams g = {};
   int bkb = 0, smem = 0;
   const double ns = plan_split(p, c.sm_count > 0 ? c.sm_count : 148, g, bkb, smem);
-  return ns < 0 ? -1 : 3400.0 + ns;
+  if (ns < 0 || !g.conv) return ns < 0 ? -1 : 3400.0 + ns;
+  // a spatial convolution waits for getting its boxes on their way, 400 to 480 ns a slab (fitted to 466 calls of 4 to 100 us)
+  const double slabs = (bkb == 128 ? 403.0 : (bkb == 64 ? 463.0 : 483.0)) * g.slabs_per;
+  return 2470.0 + (1.33 * ns > slabs ? 1.33 * ns : slabs);
 }
 
 bool launch_igemm_split(Context &c, const ConvProblem &p)

@@ -816,12 +816,15 @@ bool igemm_tc_whole_rows(const Context &c, const ConvProblem &p)
   return p.Cout * fold % 16 == 0;
 }
 
+// bytes of a slab of K, columns of a tile
+static int slab_bytes(const ConvProblem &p) { return igemm_is_plain(p) || p.Cin % 128 == 0 ? 128 : (p.Cin % 64 == 0 ? 64 : 32); }
+static int tile_columns(const ConvProblem &p) { return p.Cout <= 64 ? 64 : (p.Cout <= 128 || p.ky * p.kx * p.Cin <= 256 ? 128 : 256); }
+
 int igemm_tc_tiles(const Context &c, const ConvProblem &p, bool *few)
 {
   const int sms = c.sm_count > 0 ? c.sm_count : 148;
   const bool plain = igemm_is_plain(p);
-  const int bkb = plain ? 128 : (p.Cin % 128 == 0 ? 128 : (p.Cin % 64 == 0 ? 64 : 32));
-  const int K = p.ky * p.kx * p.Cin, bn = p.Cout <= 64 ? 64 : (p.Cout <= 128 || K <= 256 ? 128 : 256);
+  const int bkb = slab_bytes(p), K = p.ky * p.kx * p.Cin, bn = tile_columns(p);
   long long m = ((long long)p.B * p.Ho * p.Wo + BM - 1) / BM;
   if (!plain) {
     const int l = pick_patch_width_log2(p.Ho, p.Wo, p.sx, p.sy);
@@ -830,6 +833,16 @@ int igemm_tc_tiles(const Context &c, const ConvProblem &p, bool *few)
   const long long tiles = m * ((p.Cout + bn - 1) / bn);
   *few = tiles * 8 <= sms + 8 && (K + bkb - 1) / bkb >= 8;
   return (int)(tiles < 0x7fffffff ? tiles : 0x7fffffff);
+}
+
+// Fitted to 270 calls of 3 to 200 us (standard deviation 5 %): getting a slab on its way costs the producer 190 to 340 ns,
+// its bytes 2.3 ns a KB, and the tile's drain 340 ns per 64 columns.
+double igemm_tc_spatial_estimate(const Context &c, const ConvProblem &p)
+{
+  bool few;
+  const int sms = c.sm_count > 0 ? c.sm_count : 148, tiles = igemm_tc_tiles(c, p, &few), bkb = slab_bytes(p), bn = tile_columns(p);
+  const double slabs = (p.ky * p.kx * p.Cin + bkb - 1) / bkb, rounds = tiles / sms + (tiles % sms != 0);
+  return 2790 + rounds * (slabs * ((bkb == 128 ? 343 : (bkb == 64 ? 234 : 188)) + 0.0023 * bkb * (BM + bn)) + 5.3 * bn);
 }
 
 bool launch_igemm_tc(Context &c, const ConvProblem &p)

@@ -272,6 +272,7 @@ double conv_halo_tc_estimate(const Context &c, const ConvProblem &p);
 bool launch_conv_halo_tc(Context &c, const ConvProblem &p);
 // any channel count and alignment on the tensor cores, the im2col rows gathered by the warps
 bool conv_gather_tc_supported(const ConvProblem &p);
+double conv_gather_tc_estimate(const Context &c, const ConvProblem &p);       // ns, -1 where it does not take the problem
 bool launch_conv_gather_tc(Context &c, const ConvProblem &p);
 bool conv_smallcin_tc_supported(const ConvProblem &p);
 bool launch_conv_smallcin_tc(Context &c, const ConvProblem &p);
@@ -284,6 +285,7 @@ bool igemm_tc_whole_rows(const Context &c, const ConvProblem &p);
 // m-tiles x n-tiles that kernel cuts the problem into, and whether these are so few that it leaves the GPU idle over a
 // reduction of eight slabs or more
 int igemm_tc_tiles(const Context &c, const ConvProblem &p, bool *few);
+double igemm_tc_spatial_estimate(const Context &c, const ConvProblem &p);     // ns of a spatial kernel with whole rows
 // the same GEMM computed by pairs of SMs (tcgen05 cta_group::2), for wide layers with a long reduction
 bool igemm_tc2_supported(const Context &c, const ConvProblem &p);
 bool launch_igemm_tc2(Context &c, const ConvProblem &p);

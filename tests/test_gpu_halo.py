@@ -52,9 +52,10 @@ def test_modes(bits, relu, bn, gpu, restatement):
 def test_shapes(H, W, Cin, Cout, kernel, pads, batch, strides, gpu, restatement):
     c = wl.conv_case(111, H, W, Cin, Cout, kernel=kernel, pads=pads, strides=strides, batch=batch, out_shift=12)
     got = gpu.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c))
-    # four boxes a chunk, and the weights beside them leave no room for two sets, or too many cuts of the channels
-    left = strides == (2, 2) and (H, W, Cin) in ((16, 8, 128), (24, 24, 128), (16, 24, 256))
-    assert api.last_kernel() == ("igemm_tc_kernel" if left else KERNEL)
+    # where the boxes of a stride or the cuts of the channels leave another kernel ahead, or do not fit
+    others = {(28, 28, 128): ((2, 1), (1, 2)), (16, 8, 128): ((2, 2),), (20, 40, 128): ((1, 1),), (24, 24, 128): ((2, 2), (2, 1), (1, 2)),
+              (16, 24, 256): ((2, 2), (2, 1)), (16, 24, 192): ((2, 2),)}
+    assert (api.last_kernel() == KERNEL) == (strides not in others.get((H, W, Cin), ()))
     x = c["x"]
     for b in (0, batch // 2, batch - 1):
         same(got[b:b + 1], restatement.conv(32, x[b:b + 1], c["w"], c["k"], c["lam"], **conv_kw(c)))
