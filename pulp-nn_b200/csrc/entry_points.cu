@@ -457,7 +457,9 @@ static FewTiles few_tiles_form(const Context &c, const ConvProblem &p)
 // Shapes that igemm_tc takes but the gathering kernel runs faster. Output rows that are no whole 16-byte pieces, which
 // igemm_tc stores byte by byte (us, igemm_tc / gather): 56x56x128 -> 100 at batch 64 177 / 26, 28x28x256 -> 250 at batch
 // 32 78 / 12, 18x18x32 -> 77 at batch 59 19.6 / 6.6, 3x3 28x28x64 -> 100 at batch 16 19.7 / 8.6 (equal only for 3x3
-// 14x14x256 -> 77: 20.6 / 21.6). Spatial kernels on channel slabs of 32 bytes, up to 192 output channels: 56x56x96 -> 96
+// 14x14x256 -> 77: 20.6 / 21.6) -- unless these are few: igemm_tc has the shorter start (24 vectors of 48 -> 3 2.8 / 4.8,
+// 128 -> 2 over 97x97 pixels 3.2 / 3.8; of 173 such calls of up to 1700 values a tile and five slabs, 7 are better off in
+// the gathering kernel; beyond 2200 values or eight slabs the lines cross). Spatial kernels on channel slabs of 32 bytes, up to 192 output channels: 56x56x96 -> 96
 // at batch 32 43.9 / 27.4, 28x28x160 -> 160 24.9 / 18.8, 56x56x32 -> 64 at batch 64 29.5 / 22.6, 28x28x32 -> 128 11.7 /
 // 11.8; 32 -> 256 13.3 / 16.9, 224 -> 224 18.4 / 19.4. Slabs of 64 bytes, up to 64 channels and enough tiles: 56x56x64
 // -> 64 at batch 64 36.4 / 30.8, at batch 16 13.0 / 12.5; one image 5.3 / 6.7. (The spatial kernels whose weights fit an
@@ -465,7 +467,7 @@ static FewTiles few_tiles_form(const Context &c, const ConvProblem &p)
 static bool gather_first(const Context &c, const ConvProblem &p)
 {
   if (c.opt_split_k != 0 || !conv_gather_tc_supported(p)) return false;
-  if (!igemm_tc_whole_rows(c, p)) return true;
+  if (!igemm_tc_whole_rows(c, p)) return !igemm_tc_few_values(p);
   if (p.ky * p.kx == 1 || p.Cin % 128 == 0) return false;
   if (p.Cin % 64 != 0) return p.Cout <= 192;
   bool few;

@@ -835,6 +835,13 @@ int igemm_tc_tiles(const Context &c, const ConvProblem &p, bool *few)
   return (int)(tiles < 0x7fffffff ? tiles : 0x7fffffff);
 }
 
+bool igemm_tc_few_values(const ConvProblem &p)
+{
+  const long long rows = (long long)p.B * p.Ho * p.Wo;
+  const int bn = tile_columns(p), bkb = slab_bytes(p);
+  return (rows < BM ? rows : BM) * (p.Cout < bn ? p.Cout : bn) <= 1700 && (p.ky * p.kx * p.Cin + bkb - 1) / bkb <= 5;
+}
+
 // Fitted to 270 calls of 3 to 200 us (standard deviation 5 %): getting a slab on its way costs the producer 190 to 340 ns,
 // its bytes 2.3 ns a KB, and the tile's drain 340 ns per 64 columns.
 double igemm_tc_spatial_estimate(const Context &c, const ConvProblem &p)

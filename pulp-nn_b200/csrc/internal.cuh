@@ -282,6 +282,8 @@ bool igemm_tc_supported(const Context &c, const ConvProblem &p);
 bool launch_igemm_tc(Context &c, const ConvProblem &p);
 // whether its output rows are whole 16-byte pieces; otherwise it stores byte by byte
 bool igemm_tc_whole_rows(const Context &c, const ConvProblem &p);
+// whether a tile has so few values, behind so short a reduction, that storing them byte by byte does not matter
+bool igemm_tc_few_values(const ConvProblem &p);
 // m-tiles x n-tiles that kernel cuts the problem into, and whether these are so few that it leaves the GPU idle over a
 // reduction of eight slabs or more
 int igemm_tc_tiles(const Context &c, const ConvProblem &p, bool *few);

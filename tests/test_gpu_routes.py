@@ -32,3 +32,19 @@ def test_spatial_kernels(B, H, W, Cin, Cout, kernel, strides, took, gpu, restate
     assert api.last_kernel() == took
     c["x"] = c["x"][-1:]
     same(got[-1:], restatement.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
+
+
+# rows of no whole 16-byte pieces, few and many values a tile (the line: 1700 values, five slabs)
+@pytest.mark.parametrize("B,K,N,took", [(24, 48, 3, "igemm_tc_kernel"), (1, 32, 38, "igemm_tc_kernel"), (300, 320, 13, "igemm_tc_kernel"),
+                                        (2815, 32, 2, "igemm_tc_kernel"), (300, 320, 14, "conv_gather_tc_kernel"),
+                                        (24, 16, 77, "conv_gather_tc_kernel")])
+def test_ragged_rows(B, K, N, took, gpu, restatement):
+    c = wl.linear_case(131, K, N, batch=B, with_bias=True)
+    kw = dict(bias=c["bias"], out_mult=c["out_mult"], out_shift=9, relu=c["relu"], bn=c["bn"])
+    got = gpu.linear(32, c["x"], c["w"], c["k"], c["lam"], **kw)
+    assert api.last_kernel() == took
+    same(got, restatement.linear(32, c["x"], c["w"], c["k"], c["lam"], **kw))
+    if N % 4:
+        got = gpu.linear_out_32(c["x"], c["w"], bias32=c["bias32"])
+        assert api.last_kernel() == took
+        same(got, restatement.linear_out_32(c["x"], c["w"], bias32=c["bias32"]))
