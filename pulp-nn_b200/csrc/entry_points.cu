@@ -512,6 +512,11 @@ bool launch_conv(Context &c, const ConvProblem &p)
   // -> 16: 6.5 against 7.5), otherwise it leaves the GPU idle (16 of 28x28x1, 5x5: 5.7 against 4.7; 16 of 96x96x3 ->
   // 24: 77 against 13).
   if (!c.opt_force_generic && conv_smallcin_supported(p) && p.B >= 48 && p.Ho * p.Wo <= 1024) return launch_conv_smallcin(c, p);
+  // 32-bit outputs of a reduction of at most 44 terms: the dp4a kernel starts sooner and stores its words as they are (2
+  // vectors of 4 -> 4 2.8 us against 4.9, 58 of 8 -> 1896 4.0 / 5.4; of 30 such calls two, of 35 and 41 terms over 900
+  // vectors and more, are better off in the gathering kernel), while its tiles of 64x64 are a single round.
+  const long long tiles64 = ((long long)p.B * p.Ho * p.Wo + 63) / 64 * ((p.Cout + 63) / 64);
+  if (p.epi.mode == EPI_RAW32 && p.ky * p.kx * p.Cin <= 44 && tiles64 <= (c.sm_count > 0 ? c.sm_count : 148)) return launch_conv_generic(c, p);
   // Every other channel count and alignment: 48x48x20 -> 40 at batch 32 12.3 us against 33.6 in the dp4a kernel,
   // 56x56x181 -> 250 at batch 8 55 against 719, a 1001 -> 1000 linear layer 6.6 against 52, and 3.8 against 7.3 for the
   // smallest (7x7x16 -> 16, one image). What is left to the dp4a kernel are tensors beyond 32-bit offsets.

@@ -66,7 +66,7 @@ def test_pointwise_and_linear(cin, cout, gpu, restatement):
     for batch in (1, 130):
         c = wl.linear_case(73, cin, cout, batch=batch, with_bias=True)
         got = gpu.linear_out_32(c["x"], c["w"], bias32=c["bias32"])
-        assert api.last_kernel() == KERNEL
+        assert api.last_kernel() == (KERNEL if cin > 44 else "conv_generic_kernel")
         same(got, restatement.linear_out_32(c["x"], c["w"], bias32=c["bias32"]))
 
 

@@ -48,3 +48,13 @@ def test_ragged_rows(B, K, N, took, gpu, restatement):
         got = gpu.linear_out_32(c["x"], c["w"], bias32=c["bias32"])
         assert api.last_kernel() == took
         same(got, restatement.linear_out_32(c["x"], c["w"], bias32=c["bias32"]))
+
+
+# 32-bit outputs of short reductions of no whole 16 bytes (the line: 44 terms, one round of 64x64 tiles)
+@pytest.mark.parametrize("B,K,N,took", [(2, 4, 4, "conv_generic_kernel"), (58, 8, 1896, "conv_generic_kernel"), (70, 44, 33, "conv_generic_kernel"),
+                                        (70, 45, 33, "conv_gather_tc_kernel"), (2500, 12, 300, "conv_gather_tc_kernel")])
+def test_short_reductions(B, K, N, took, gpu, restatement):
+    c = wl.linear_case(132, K, N, batch=B, with_bias=True)
+    got = gpu.linear_out_32(c["x"], c["w"], bias32=c["bias32"])
+    assert api.last_kernel() == took
+    same(got, restatement.linear_out_32(c["x"], c["w"], bias32=c["bias32"]))
