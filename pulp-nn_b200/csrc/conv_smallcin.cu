@@ -12,6 +12,8 @@
 // channel whose bytes beyond kx*ch_in are zero, so whatever the third word drags in is ignored.
 // A thread computes two output pixels for all 32 output channels: weights are read from shared
 // memory as broadcast 16-byte loads (4 channels at a time), one dp4a per channel and word.
+#include <cmath>
+
 #include "internal.cuh"
 
 namespace pulpnn {
@@ -201,6 +203,38 @@ bool conv_smallcin_supported(const ConvProblem &p)
   return fixed_bytes(p) + (size_t)p.ky * staged_pitch(p) <= 48 * 1024;
 }
 
+// output rows of a strip
+static int strip_rows(const ConvProblem &p)
+{
+  const size_t fixed = fixed_bytes(p), pitch = staged_pitch(p);
+  // strip height: shared memory under 48 KB, and a pixel-pair count close to a multiple of 256
+  int best = 1; double best_waste = 1e9;
+  for (int ro = 1; ro <= p.Ho && ro <= 64; ro++) {
+    const int rin = (ro - 1) * p.sy + p.ky;
+    if (fixed + (size_t)rin * pitch > 46 * 1024) break;
+    const int pairs = (ro * p.Wo + 1) / 2;
+    const int iters = (pairs + 255) / 256;
+    const double waste = (double)iters * 256 / pairs + 0.25 * (p.ky - p.sy > 0 ? (double)(p.ky - p.sy) / (ro * p.sy) : 0.0);
+    if (waste < best_waste - 1e-9) { best_waste = waste; best = ro; }
+  }
+  return best;
+}
+
+// Fitted to 500 calls of 2 to 380 us (standard deviation 9 %): two CTAs of an SM, each staging its rows (words, or bytes
+// where rows are no whole words), computing 512 pixels at a time and storing them (bytes where the channels are no whole
+// 16-byte pieces, which a warp's lanes scatter over as many sectors). A CTA with the SM to itself takes 0.62 of that.
+double conv_smallcin_estimate(const Context &c, const ConvProblem &p)
+{
+  const int sms = c.sm_count > 0 ? c.sm_count : 148, rows = strip_rows(p);
+  const double ctas = (double)p.B * ((p.Ho + rows - 1) / rows), pairs = (rows * p.Wo + 1) / 2;
+  const bool words = p.W * p.Cin % 4 == 0 && (reinterpret_cast<uintptr_t>(p.in) & 3) == 0;
+  const bool pieces = p.Cout % 16 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+  const double stage = (words ? 0.245 : 0.56) * ((rows - 1) * p.sy + p.ky) * staged_pitch(p);
+  const double cta = 108 + stage + ceil(pairs / 256) * (1063 + 491 * p.ky) + (pieces ? 0 : pairs / 256 * 21.2 * p.Cout * p.Cout);
+  const double waves = ctas / (2 * sms) > 1 ? 0.5 * (ceil(ctas / (2 * sms)) + ctas / (2 * sms)) : 1;
+  return 2070 + waves * cta * (ctas > sms ? 1 : 0.62);
+}
+
 bool launch_conv_smallcin(Context &c, const ConvProblem &p)
 {
   SmallParams g;
@@ -211,20 +245,10 @@ bool launch_conv_smallcin(Context &c, const ConvProblem &p)
   g.vec_rows = (g.row_bytes % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.in) & 3) == 0);
   g.vec_store = (p.Cout % 16 == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
   if (p.Cout == CO && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0) g.vec_store = 2;
-  const size_t fixed = fixed_bytes(p);
-  // strip height: shared memory under 48 KB, and a pixel-pair count close to a multiple of 256
-  int best = 1; double best_waste = 1e9;
-  for (int ro = 1; ro <= p.Ho && ro <= 64; ro++) {
-    const int rin = (ro - 1) * p.sy + p.ky;
-    if (fixed + (size_t)rin * g.pitch > 46 * 1024) break;
-    const int pairs = (ro * p.Wo + 1) / 2;
-    const int iters = (pairs + 255) / 256;
-    const double waste = (double)iters * 256 / pairs + 0.25 * (p.ky - p.sy > 0 ? (double)(p.ky - p.sy) / (ro * p.sy) : 0.0);
-    if (waste < best_waste - 1e-9) { best_waste = waste; best = ro; }
-  }
+  const int best = strip_rows(p);
   g.rows_out = best;
   g.rows_in = (best - 1) * p.sy + p.ky;
-  const size_t smem = fixed + (size_t)g.rows_in * g.pitch;
+  const size_t smem = fixed_bytes(p) + (size_t)g.rows_in * g.pitch;
   dim3 grid((unsigned)((p.Ho + best - 1) / best), (unsigned)p.B);
   switch (p.epi.mode) {
     case EPI_NONE: conv_smallcin_kernel<EPI_NONE><<<grid, 256, smem, c.stream>>>(g); break;

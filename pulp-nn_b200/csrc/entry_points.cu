@@ -507,11 +507,14 @@ bool launch_conv(Context &c, const ConvProblem &p)
     return launch_igemm_tc2(c, p);
   if (!c.opt_force_generic && igemm_tc_supported(c, p)) return gather_first(c, p) ? launch_conv_gather_tc(c, p) : launch_igemm_tc(c, p);
   if (!c.opt_force_generic && conv_smallcin_tc_supported(p)) return launch_conv_smallcin_tc(c, p);
-  // First layers that the kernel above does not take. conv_smallcin walks the strips of an image in one CTA each:
-  // with many small images it beats the gathering kernel (64 images of 28x28x1 -> 16: 4.5 against 6.9 us, of 32x32x3
-  // -> 16: 6.5 against 7.5), otherwise it leaves the GPU idle (16 of 28x28x1, 5x5: 5.7 against 4.7; 16 of 96x96x3 ->
-  // 24: 77 against 13).
-  if (!c.opt_force_generic && conv_smallcin_supported(p) && p.B >= 48 && p.Ho * p.Wo <= 1024) return launch_conv_smallcin(c, p);
+  // First layers that the kernel above does not take. conv_smallcin starts sooner and walks the strips of an image in one
+  // CTA each: it is faster for the smallest calls and where strips fill the GPU (us, this kernel / gathering: 36 pixels of 4
+  // -> 32 channels 3.4 / 4.9, 21 of 575x291x1 -> 16 130 / 210, 64 of 28x28x1 -> 16 4.5 / 6.9; 16 of 28x28x1, 5x5, 5.7 / 4.7,
+  // 16 of 96x96x3 -> 24 77 / 13). Over 500 calls the estimates are 1 % behind the faster of the two, by 5 % in 33 of them.
+  if (!c.opt_force_generic && conv_smallcin_supported(p)) {
+    const double gather = conv_gather_tc_estimate(c, p);
+    if (gather < 0 || conv_smallcin_estimate(c, p) < gather) return launch_conv_smallcin(c, p);
+  }
   // 32-bit outputs of a reduction of at most 44 terms: the dp4a kernel starts sooner and stores its words as they are (2
   // vectors of 4 -> 4 2.8 us against 4.9, 58 of 8 -> 1896 4.0 / 5.4; of 30 such calls two, of 35 and 41 terms over 900
   // vectors and more, are better off in the gathering kernel), while its tiles of 64x64 are a single round.
@@ -521,8 +524,6 @@ bool launch_conv(Context &c, const ConvProblem &p)
   // 56x56x181 -> 250 at batch 8 55 against 719, a 1001 -> 1000 linear layer 6.6 against 52, and 3.8 against 7.3 for the
   // smallest (7x7x16 -> 16, one image). What is left to the dp4a kernel are tensors beyond 32-bit offsets.
   if (!c.opt_force_generic && conv_gather_tc_supported(p)) return launch_conv_gather_tc(c, p);
-  // (first layers among those have a kernel of their own, whatever the batch)
-  if (!c.opt_force_generic && conv_smallcin_supported(p)) return launch_conv_smallcin(c, p);
   return launch_conv_generic(c, p);
 }
 

@@ -277,6 +277,7 @@ bool launch_conv_gather_tc(Context &c, const ConvProblem &p);
 bool conv_smallcin_tc_supported(const ConvProblem &p);
 bool launch_conv_smallcin_tc(Context &c, const ConvProblem &p);
 bool conv_smallcin_supported(const ConvProblem &p);
+double conv_smallcin_estimate(const Context &c, const ConvProblem &p);        // ns of a problem it takes
 bool launch_conv_smallcin(Context &c, const ConvProblem &p);
 bool igemm_tc_supported(const Context &c, const ConvProblem &p);
 bool launch_igemm_tc(Context &c, const ConvProblem &p);

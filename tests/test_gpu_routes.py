@@ -58,3 +58,18 @@ def test_short_reductions(B, K, N, took, gpu, restatement):
     got = gpu.linear_out_32(c["x"], c["w"], bias32=c["bias32"])
     assert api.last_kernel() == took
     same(got, restatement.linear_out_32(c["x"], c["w"], bias32=c["bias32"]))
+
+
+# first layers: the kernel that walks strips of an image, and the gathering one where its strips leave the GPU idle
+@pytest.mark.parametrize("B,H,W,Cin,Cout,k,took", [
+    (1, 6, 6, 4, 32, 1, "conv_smallcin_kernel"), (21, 575, 291, 1, 16, 3, "conv_smallcin_kernel"), (64, 28, 28, 1, 16, 3, "conv_smallcin_kernel"),
+    (1, 5, 5, 3, 32, 2, "conv_smallcin_kernel"), (16, 96, 96, 3, 24, 3, "conv_gather_tc_kernel"), (16, 28, 28, 1, 16, 5, "conv_gather_tc_kernel"),
+    (1, 1, 4500, 3, 16, 4, "conv_gather_tc_kernel")])
+def test_first_layers(B, H, W, Cin, Cout, k, took, gpu, restatement):
+    p = k // 2
+    kernel = (1, k) if H == 1 else (k, k)
+    c = wl.conv_case(133, H, W, Cin, Cout, kernel=kernel, pads=(p if H > 1 else 0,) * 2 + (p, p), batch=B, out_shift=9, with_bias=True)
+    got = gpu.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c))
+    assert api.last_kernel() == took
+    c["x"] = c["x"][-1:]
+    same(got[-1:], restatement.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
