@@ -1,9 +1,9 @@
 // depthwise_planes.cu -- 3x3 and 5x5 depthwise convolution, stride 1 or 2, of ANY channel count, row
 // length and alignment, from HWC or CHW input (arithmetic of 32bit/src/pulp_nn_depthwise_generic.c:133-180).
 //
-// A CTA takes one image, a group of 32 (16) channels and a band of output rows. It stages the input rows
-// of the band in shared memory as one PLANE per channel, [channel][row][x + padding_left], zeros outside
-// the image: HWC input through 4x4 byte transposes (four pixels x four channels), CHW input as it lies.
+// A CTA takes one image, a group of 32 (16) channels and a band of output rows, cut into strips of columns
+// where bands alone are too large or too few. It stages the input rows of the band in shared memory as one
+// PLANE per channel, [channel][row][x - first column it reads], zeros outside the image: HWC input through 4x4 byte transposes (four pixels x four channels), CHW input as it lies.
 // A lane is a channel, so a warp stores runs of 32 bytes of the HWC output and an odd pitch in words
 // keeps the lanes on different banks. A lane computes four adjacent output columns of R rows: their
 // windows lie in two (stride 1) or three (stride 2) aligned words of a plane row, and a filter row costs
@@ -25,7 +25,8 @@ namespace pulpnn {
 namespace {
 
 constexpr int DT = 256;
-constexpr int PLANES_SMEM = 200 * 1024;      // planes and expanded filter rows of a CTA
+constexpr int PLANES_BAND = 48 * 1024;       // planes of a CTA: four CTAs share an SM
+constexpr int PLANES_SMEM = PLANES_BAND + 5 * 4 * 2 * 32 * 4;      // and its expanded filter rows
 
 struct PlanesParams {
   DepthwiseProblem p;
@@ -34,8 +35,9 @@ struct PlanesParams {
   int plane;                    // bytes of a plane, an odd number of words
   int words;                    // HWC: channels in whole aligned words
   int quads;                    // groups of four output columns
-  FastDiv by_groups, by_bands;
-  FastDiv by_qw, by_per, by_quads;   // words (CHW: 16-byte pieces) of a plane row, of a plane; quads
+  int strips, sq;               // strips of sq such groups
+  FastDiv by_groups, by_bands, by_strips;
+  FastDiv by_qw, by_per, by_sq; // words (CHW: 16-byte pieces) of a plane row, of a plane; sq
 };
 
 __device__ __forceinline__ unsigned prmt_b(unsigned a, unsigned b, unsigned sel)
@@ -45,7 +47,9 @@ __device__ __forceinline__ unsigned prmt_b(unsigned a, unsigned b, unsigned sel)
   return d;
 }
 
-template <int MODE, int K, int S, int CG>
+// STRIPS: more than one strip (as a branch of its own the check of the last strip's groups costs the 5x5 layers of one
+// strip 2.5 %)
+template <int MODE, int K, int S, int CG, bool STRIPS>
 __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_constant__ PlanesParams g)
 {
   constexpr int R = S == 1 ? 4 : 2;                         // output rows of a lane
@@ -55,10 +59,11 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
   const DepthwiseProblem &p = g.p;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int t0 = g.by_groups.div((int)blockIdx.x), grp = (int)blockIdx.x - t0 * g.groups;
-  const int b = g.by_bands.div(t0), band = t0 - b * g.bands;
+  const int t1 = STRIPS ? g.by_strips.div(t0) : t0, xq0 = STRIPS ? (t0 - t1 * g.strips) * g.sq : 0;
+  const int b = g.by_bands.div(t1), band = t1 - b * g.bands;
   const int c0 = grp * CG, nch = min(CG, p.C - c0);
   const int oy0 = band * g.band;
-  const int iy0 = oy0 * S - p.pt;
+  const int iy0 = oy0 * S - p.pt, ix0 = (STRIPS ? 4 * S * xq0 : 0) - p.pl;
   const int qw = g.row_pitch >> 2;                          // words of a plane row
 
   pdl_wait();
@@ -105,7 +110,7 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
       for (int u = 0; u < U; u++) {
         const int it = it0 + u * STEP;
         const int row = g.by_qw.div(it), q = it - row * qw;
-        const int iy = iy0 + row, ix = 4 * q - p.pl;
+        const int iy = iy0 + row, ix = ix0 + 4 * q;
         const bool ok = it < items && (unsigned)iy < (unsigned)p.H && left > 0;
         at[u] = (iy * p.W + ix) * p.C + c0 + 4 * cq + lead;
         dst[u] = it < items ? 4 * cq * g.plane + row * g.row_pitch + 4 * q : -1;
@@ -171,7 +176,7 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
         const int it = it0 + u * DT;
         const int ch = g.by_per.div(it), rq = it - ch * per;
         const int row = g.by_qw.div(rq), q = rq - row * pw;
-        const int iy = iy0 + row, ix = 16 * q - p.pl;
+        const int iy = iy0 + row, ix = ix0 + 16 * q;
         from[u] = max(-ix, 0);
         to[u] = it < items && (unsigned)iy < (unsigned)p.H && from[u] < 16 ? min(p.W - ix, 16) : 0;
         t[u].fetch(in, first + (ch * p.H + iy) * p.W + ix, to[u] > 0);
@@ -223,11 +228,11 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
 
   // ---- compute: a unit is four columns x R rows of the warp's channels ------------------------------
   const int rows = min(g.band, p.Ho - oy0);
-  const int units = ((rows + R - 1) / R) * g.quads;
+  const int units = ((rows + R - 1) / R) * g.sq;
   const uint8_t *mine = planes + (size_t)cl * g.plane;
   uint8_t *out = p.out + (size_t)b * p.Ho * p.Wo * p.C;
   for (int u = warp * (32 / CG) + sub; u < units; u += (DT / 32) * (32 / CG)) {
-    const int rb = g.by_quads.div(u), xq = u - rb * g.quads;
+    const int rb = g.by_sq.div(u), xq = u - rb * g.sq;
     int acc[R][4];
 #pragma unroll
     for (int r = 0; r < R; r++)
@@ -251,13 +256,13 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
         }
       }
     }
-    const int oy = oy0 + rb * R, ox = xq * 4;
+    const int oy = oy0 + rb * R, ox = (STRIPS ? xq0 + xq : xq) * 4;
     const bool whole = ox + 4 <= p.Wo;
     unsigned o = (unsigned)((oy * p.Wo + ox) * p.C + c);
 #pragma unroll
     for (int r = 0; r < R; r++, o += (unsigned)(p.Wo * p.C)) {
       const unsigned w = pack4_sat_u8(scaled(acc[r][0]), scaled(acc[r][1]), scaled(acc[r][2]), scaled(acc[r][3]));
-      if (cl >= nch || oy + r >= p.Ho) continue;
+      if (cl >= nch || oy + r >= p.Ho || (STRIPS && ox >= p.Wo)) continue;
       out[o] = (uint8_t)w;
       if (whole) {
         out[o + p.C] = (uint8_t)(w >> 8);
@@ -271,36 +276,36 @@ __global__ void __launch_bounds__(DT) depthwise_planes_kernel(const __grid_const
   }
 }
 
-template <int MODE, int K, int S, int CG>
+template <int MODE, int K, int S, int CG, bool STRIPS>
 bool launch_planes(Context &c, const PlanesParams &g, int smem)
 {
-  auto kern = depthwise_planes_kernel<MODE, K, S, CG>;
+  auto kern = depthwise_planes_kernel<MODE, K, S, CG, STRIPS>;
   static PerDeviceInt attr_set;
   if (!attr_set.get(c.device)) {
     if (!cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PLANES_SMEM), "cudaFuncSetAttribute(depthwise_planes)"))
       return false;
     attr_set.set(c.device, 1);
   }
-  const cudaError_t le = launch_pdl(kern, dim3((unsigned)(g.groups * g.bands * g.p.B)), dim3(DT), (size_t)smem, c.stream, g);
+  const cudaError_t le = launch_pdl(kern, dim3((unsigned)(g.groups * g.strips * g.bands * g.p.B)), dim3(DT), (size_t)smem, c.stream, g);
   count_launch("depthwise_planes_kernel");
   return cuda_ok(le, "depthwise_planes launch") && cuda_ok(cudaGetLastError(), "depthwise_planes launch");
 }
 
-template <int MODE, int CG>
+template <int MODE, int CG, bool STRIPS>
 bool launch_planes_ks(Context &c, const PlanesParams &g, int smem)
 {
-  if (g.p.kx == 3) return g.p.sx == 1 ? launch_planes<MODE, 3, 1, CG>(c, g, smem) : launch_planes<MODE, 3, 2, CG>(c, g, smem);
-  return g.p.sx == 1 ? launch_planes<MODE, 5, 1, CG>(c, g, smem) : launch_planes<MODE, 5, 2, CG>(c, g, smem);
+  if (g.p.kx == 3) return g.p.sx == 1 ? launch_planes<MODE, 3, 1, CG, STRIPS>(c, g, smem) : launch_planes<MODE, 3, 2, CG, STRIPS>(c, g, smem);
+  return g.p.sx == 1 ? launch_planes<MODE, 5, 1, CG, STRIPS>(c, g, smem) : launch_planes<MODE, 5, 2, CG, STRIPS>(c, g, smem);
 }
 
 template <int MODE>
 bool launch_planes_mode(Context &c, const PlanesParams &g, int cg, int smem)
 {
-  return cg == 16 ? launch_planes_ks<MODE, 16>(c, g, smem) : launch_planes_ks<MODE, 32>(c, g, smem);
+  if (g.strips > 1) return cg == 16 ? launch_planes_ks<MODE, 16, true>(c, g, smem) : launch_planes_ks<MODE, 32, true>(c, g, smem);
+  return cg == 16 ? launch_planes_ks<MODE, 16, false>(c, g, smem) : launch_planes_ks<MODE, 32, false>(c, g, smem);
 }
 
-// lays the work out; false when not even one band of R rows and the filter rows fit shared memory or the grid is too
-// large
+// lays the work out; false when the offsets or the grid are too large
 bool configure(const DepthwiseProblem &p, int sms, PlanesParams &g, int &cg, int &smem)
 {
   const int S = p.sx, K = p.kx, R = S == 1 ? 4 : 2;
@@ -308,36 +313,47 @@ bool configure(const DepthwiseProblem &p, int sms, PlanesParams &g, int &cg, int
   cg = p.C <= 16 ? 16 : 32;
   g.groups = (p.C + cg - 1) / cg;
   g.quads = (p.Wo + 3) / 4;
-  long long pitch = (long long)(g.quads - 1) * 4 * S + 4 * (((3 * S + K - 1) >> 2) + 1);
-  if (!p.in_is_hwc) pitch = (pitch + 15) & ~15LL;           // rows are staged in 16-byte pieces
   g.words = p.C % 4 == 0 && (reinterpret_cast<uintptr_t>(p.in) & 3) == 0;
-  auto plane_of = [&](int band) {
-    long long w = ((long long)(band - 1) * S + K) * (pitch / 4);
+  auto pitch_of = [&](int sq) {
+    const long long pitch = (long long)(sq - 1) * 4 * S + 4 * (((3 * S + K - 1) >> 2) + 1);
+    return p.in_is_hwc ? pitch : (pitch + 15) & ~15LL;      // CHW rows are staged in 16-byte pieces
+  };
+  auto plane_of = [&](int band, int sq) {
+    const long long w = ((long long)(band - 1) * S + K) * (pitch_of(sq) / 4);
     return (w | 1) * 4;
   };
-  // whole images while they fit 48 KB (four CTAs of an SM), shorter bands until the GPU is full
+  // whole images while they fit, shorter bands until the GPU is full
   const int rb = (p.Ho + R - 1) / R;
   int blocks = rb;
-  while (blocks > 1 && (plane_of(blocks * R) * cg > 48 * 1024 || (long long)p.B * g.groups * ((rb + blocks - 1) / blocks) < 2LL * sms))
+  while (blocks > 1 && (plane_of(blocks * R, g.quads) * cg > PLANES_BAND || (long long)p.B * g.groups * ((rb + blocks - 1) / blocks) < 2LL * sms))
     blocks = (blocks + 1) / 2;
   g.band = blocks * R;
+  g.bands = (p.Ho + g.band - 1) / g.band;
+  // Strips of no fewer than 32 columns where bands of R rows are still too large, or too few for the GPU: one row of 1038
+  // pixels of 154 channels was staged and computed by five CTAs, in 23.7 us against 3.1 in strips.
+  const long long ctas = (long long)p.B * g.groups * g.bands;
+  long long n = ctas < 2LL * sms ? (2LL * sms + ctas - 1) / ctas : 1;
+  if (n > (g.quads + 7) / 8) n = (g.quads + 7) / 8;
+  g.sq = (int)((g.quads + n - 1) / n);
+  while (g.sq > 8 && plane_of(g.band, g.sq) * cg > PLANES_BAND) g.sq = (g.sq + 1) / 2;
+  g.strips = (g.quads + g.sq - 1) / g.sq;
   const int filters = K * (4 / S) * 2 * cg * 4;
-  if (plane_of(g.band) * cg + filters > PLANES_SMEM) return false;
+  if (plane_of(g.band, g.sq) * cg + filters > PLANES_SMEM) return false;
   // 32-bit offsets inside a group of channels, the rows above and below its image included
   if (((long long)cg * p.H + p.pt + g.band * S + K) * p.W > 0x7fff0000LL) return false;
   if ((long long)p.Ho * p.Wo * p.C > 0x7fff0000LL || ((long long)p.H + p.pt + g.band * S + K) * p.W * p.C > 0x7fff0000LL) return false;
-  g.bands = (p.Ho + g.band - 1) / g.band;
-  if ((long long)g.groups * g.bands * p.B > 0x7fffffffLL) return false;
-  g.row_pitch = (int)pitch;
+  if (ctas * g.strips > 0x7fffffffLL) return false;
+  g.row_pitch = (int)pitch_of(g.sq);
   g.rows_in = (g.band - 1) * S + K;
-  g.plane = (int)plane_of(g.band);
+  g.plane = (int)plane_of(g.band, g.sq);
   smem = g.plane * cg + filters;
   g.by_groups.set((unsigned)g.groups);
   g.by_bands.set((unsigned)g.bands);
+  g.by_strips.set((unsigned)g.strips);
   const int piece = p.in_is_hwc ? 4 : 16;
   g.by_qw.set((unsigned)(g.row_pitch / piece));
   g.by_per.set((unsigned)(g.rows_in * (g.row_pitch / piece)));
-  g.by_quads.set((unsigned)g.quads);
+  g.by_sq.set((unsigned)g.sq);
   return true;
 }
 

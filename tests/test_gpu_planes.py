@@ -43,22 +43,23 @@ def test_shapes(k, s, hwc, H, W, C, batch, gpu, restatement):
     same(got, restatement.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
 
 
-# the widest rows whose band and filter rows fit a CTA's shared memory, the first that do not, and the last whose band
-# alone would: each is followed by an ordinary call, which has to find nothing left over
-@pytest.mark.parametrize("k,s,hwc,H,W,C,fits", [
-    (5, 1, True, 8, 772, 20, 1), (5, 1, True, 8, 773, 20, 0), (5, 1, True, 8, 784, 40, 0), (5, 1, True, 8, 792, 20, 0),
-    (5, 1, True, 8, 793, 20, 0), (5, 1, False, 8, 764, 20, 1), (5, 1, False, 8, 776, 20, 0), (5, 1, False, 8, 780, 20, 0),
-    (5, 2, True, 6, 896, 20, 1), (5, 2, True, 6, 900, 20, 0), (5, 2, False, 6, 888, 20, 1), (5, 2, False, 6, 904, 20, 0),
-    (5, 1, True, 5, 1580, 8, 0), (3, 1, True, 4, 1044, 30, 1), (3, 1, True, 4, 1050, 30, 0), (3, 1, True, 4, 1048, 64, 0),
-    (3, 1, True, 4, 1060, 30, 0), (3, 1, False, 4, 1036, 20, 1), (3, 1, False, 4, 1044, 20, 0), (3, 1, False, 4, 1052, 20, 0),
-    (3, 2, True, 6, 1264, 30, 1), (3, 2, True, 6, 1270, 30, 0), (3, 1, True, 4, 2120, 7, 0)])
-def test_widest_rows(k, s, hwc, H, W, C, fits, gpu, restatement):
+# rows in one and in several strips of columns: the last strip whole, of one group of four columns and of a part of one;
+# images of few rows and many, bands that would not fit shared memory in one piece. Each is followed by an ordinary call,
+# which has to find nothing left over.
+@pytest.mark.parametrize("k,s,hwc,H,W,C,batch", [
+    (5, 1, True, 8, 773, 20, 1), (5, 1, True, 8, 784, 40, 1), (5, 1, False, 8, 776, 20, 1), (5, 2, True, 6, 900, 20, 1),
+    (5, 2, False, 6, 901, 20, 1), (5, 1, True, 5, 1580, 8, 1), (3, 1, True, 4, 1050, 30, 1), (3, 1, False, 4, 1052, 20, 1),
+    (3, 2, True, 6, 1270, 30, 1), (3, 1, True, 4, 2120, 7, 1), (3, 1, True, 1, 1038, 154, 1), (3, 1, True, 1, 32, 5, 3),
+    (3, 1, True, 1, 33, 5, 3), (3, 1, False, 2, 36, 17, 1), (5, 2, True, 3, 65, 6, 2), (5, 2, False, 3, 72, 33, 2),
+    (3, 2, False, 1, 130, 31, 2), (3, 1, True, 9, 300, 3, 200), (5, 1, False, 30, 700, 18, 40)])
+def test_strips_of_columns(k, s, hwc, H, W, C, batch, gpu, restatement):
     p = k // 2
-    for h, w, c, planes in ((H, W, C, fits), (9, 7, 20, 1)):
-        c = wl.depthwise_case(83, h, w, c, kernel=(k, k), strides=(s, s), pads=(p, p, p, p), out_shift=9, hwc=hwc)
+    for h, w, c, b in ((H, W, C, batch), (9, 7, 20, 1)):
+        c = wl.depthwise_case(83, h, w, c, kernel=(k, k), strides=(s, s), pads=(p, p, p, p), batch=b, out_shift=9, hwc=hwc)
         got = gpu.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c))
-        assert (api.last_kernel() == KERNEL) == bool(planes)
-        same(got, restatement.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
+        assert api.last_kernel() == KERNEL
+        c["x"] = c["x"][-1:]
+        same(got[-1:], restatement.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
 
 
 @pytest.mark.parametrize("hwc", [False, True])
