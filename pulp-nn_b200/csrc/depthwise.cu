@@ -271,12 +271,22 @@ bool launch_dw_mode(Context &c, const DepthwiseProblem &p)
 //              32x56x56x100 12.5 MB 8.3 / 11.8
 //  CHW, TMA:   16x32x32x128 4.2 MB 5.9 / 7.4, 8x112x112x32 6.4 MB 7.5 / 7.8; stride 2: 4x112x112x64 4.0 MB 5.4 / 6.7, 8 of
 //              them 8.0 MB 8.3 / 6.6
-static bool planes_first(const DepthwiseProblem &p, bool tma)
+//  One row of output, of which the plane kernel computes two or four and stages as many: TMA 1x1958x128 0.4 MB 2.6 / 2.5,
+//              1x3041x224 1.4 MB 6.4 / 3.0; registers 1x749x148 0.2 MB 2.4 / 2.8, 12x131x140 0.4 MB 3.8 / 3.0, 45x1830x16
+//              2.0 MB 5.9 / 3.3; 5x5 against the general kernel 25x101x128 0.5 MB 3.3 / 5.2, 5x2109x224 4.7 MB 17.0 / 9.7
+enum class DwOther { tma, registers, general };
+static bool planes_first(const DepthwiseProblem &p, DwOther other)
 {
   const long long bytes = (long long)p.B * p.C * ((long long)p.H * p.W + (long long)p.Ho * p.Wo);
+  const bool one_row = p.Ho == 1;
   long long kb;
-  if (!p.in_is_hwc) kb = p.sx == 1 ? 6500 : 4500;
-  else if (tma)     kb = p.H >= 28 ? 4500 : (p.H >= 14 ? 2200 : 600);
+  if (other == DwOther::general) {
+    if (!one_row || !p.in_is_hwc || p.kx < 5) return true;
+    kb = 1000;
+  }
+  else if (one_row) kb = other == DwOther::tma ? 0 : 300;
+  else if (!p.in_is_hwc) kb = p.sx == 1 ? 6500 : 4500;
+  else if (other == DwOther::tma) kb = p.H >= 28 ? 4500 : (p.H >= 14 ? 2200 : 600);
   else              kb = p.sx == 1 ? 9000 : 16000;
   return bytes <= kb * 1000;
 }
@@ -286,10 +296,10 @@ bool launch_depthwise(Context &c, const DepthwiseProblem &p)
   if (!c.opt_force_generic) {
     const bool planes = depthwise_planes_supported(p);
     const bool tma = p.in_is_hwc ? depthwise_hwc3x3_tma_supported(p) : depthwise_chw3x3_tma_supported(p);
-    if (tma && !(planes && planes_first(p, true)))
+    if (tma && !(planes && planes_first(p, DwOther::tma)))
       return p.in_is_hwc ? launch_depthwise_hwc3x3_tma(c, p) : launch_depthwise_chw3x3_tma(c, p);
-    if (depthwise_hwc3x3_supported(p) && !(planes && planes_first(p, false))) return launch_depthwise_hwc3x3(c, p);
-    if (planes) return launch_depthwise_planes(c, p);
+    if (depthwise_hwc3x3_supported(p) && !(planes && planes_first(p, DwOther::registers))) return launch_depthwise_hwc3x3(c, p);
+    if (planes && planes_first(p, DwOther::general)) return launch_depthwise_planes(c, p);
   }
   switch (p.epi.mode) {
     case EPI_NONE: return launch_dw_mode<EPI_NONE>(c, p);

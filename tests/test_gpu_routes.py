@@ -2,7 +2,7 @@
 import pytest
 
 from conftest import pulpnn
-from test_gpu_parity import conv_kw, same
+from test_gpu_parity import conv_kw, dw_kw, same
 
 pytestmark = pytest.mark.gpu
 api, wl = pulpnn.api, pulpnn.workloads
@@ -73,3 +73,18 @@ def test_first_layers(B, H, W, Cin, Cout, k, took, gpu, restatement):
     assert api.last_kernel() == took
     c["x"] = c["x"][-1:]
     same(got[-1:], restatement.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
+
+
+# depthwise layers with one row of output, of which the plane kernel computes two or four
+@pytest.mark.parametrize("B,W,C,k,s,hwc,took", [
+    (1, 1958, 128, 3, 2, True, "depthwise_hwc3x3_tma_kernel"), (15, 80, 32, 3, 1, False, "depthwise_chw3x3_tma_kernel"),
+    (1, 749, 148, 3, 1, True, "depthwise_planes_kernel"), (45, 1830, 16, 3, 2, True, "depthwise_hwc3x3_kernel"),
+    (25, 101, 128, 5, 2, True, "depthwise_planes_kernel"), (5, 2109, 224, 5, 1, True, "depthwise_generic_kernel"),
+    (24, 1643, 174, 3, 1, True, "depthwise_planes_kernel")])
+def test_one_row_depthwise(B, W, C, k, s, hwc, took, gpu, restatement):
+    p = k // 2
+    c = wl.depthwise_case(137, 1, W, C, kernel=(k, k), strides=(s, s), pads=(p, p, p, p), batch=B, out_shift=9, hwc=hwc)
+    got = gpu.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c))
+    assert api.last_kernel() == took
+    c["x"] = c["x"][-1:]
+    same(got[-1:], restatement.depthwise(32, c["x"], c["w"], c["k"], c["lam"], **dw_kw(c)))
