@@ -29,6 +29,19 @@ def test_pool(C, k, s, p, gpu, restatement):
         same(gpu.avgpool(bits, x, **q, **kw), restatement.avgpool(bits, x, **q, **kw))
 
 
+# averages of whole 16-channel pieces: four channels a thread on either side of 256 threads of sixteen an SM, sixteen beyond
+@pytest.mark.parametrize("batch", [1, 9, 10, 32])
+@pytest.mark.parametrize("k,s", [(2, 2), (3, 2), (1, 2)])
+def test_average_of_whole_pieces(batch, k, s, gpu, restatement):
+    x = np.random.default_rng(9).integers(0, 256, size=(batch, 64, 66, 64), dtype=np.uint8)
+    kw = dict(out_hw=((64 - k) // s + 1, (66 - k) // s + 1), kernel=(k, k), pads=(0, 0, 0, 0), strides=(s, s))
+    for bits, requant in ((32, 0), (32, 1), (64, 1)):
+        q = dict(lam=77, out_shift=6, out_add=130, requant=requant)
+        got = gpu.avgpool(bits, x, **q, **kw)
+        assert api.last_kernel() == "pool_kernel"
+        same(got[-1:], restatement.avgpool(bits, x[-1:], **q, **kw))
+
+
 def test_windows_that_pads_shift(gpu, restatement):
     """An average's window starts by padding_b and ends by padding_r."""
     rng = np.random.default_rng(5)
