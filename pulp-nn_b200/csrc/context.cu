@@ -101,6 +101,14 @@ void *ctx_scratch(Context &c, size_t bytes)
   return c.scratch;
 }
 
+bool ctx_scratch_at_hand(Context &c, size_t bytes)
+{
+  if (bytes <= c.scratch_cap) return true;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c.stream, &cap) != cudaSuccess) { cudaGetLastError(); return false; }
+  return cap == cudaStreamCaptureStatusNone;
+}
+
 // device word that kernels with bounded waits report into (read by pulpnn_device_status)
 int *ctx_status_word(Context &c)
 {

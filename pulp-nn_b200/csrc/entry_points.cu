@@ -427,8 +427,11 @@ void add_entry(uint8_t *a, uint8_t *b, uint8_t *out, int m1, int m2, int out_shi
 //   256 x 4096 -> 4096  17.4 / 33  / 13.0           512 x 4096 -> 4096 17.5 / 34 / 19.4          784 x 1024 -> 1024  7.7 / 9.8 / 9.2
 //   3x3, one image: 32x32x32 -> 64 8.1 / 4.4 / 7.7, 14x14x64 -> 64 8.1 / 5.4 / 7.5, 28x28x128 -> 128 10.4 / 6.6 / 6.8,
 //   7x7x512 -> 512 10.1 / 8.5 / 7.1; 14x14x256 -> 256 at batch 8 14.3 / 11.1 / 9.1, 28x28x128 -> 128 at batch 4 7.4 / 9.1 / 8.2
-enum class FewTiles { none, rows, gather, split };
-static FewTiles few_tiles_form(const Context &c, const ConvProblem &p)
+// Beyond 18000 terms the 16 slices of a split through memory (igemm_tc and a second kernel) leave the eight CTAs of a
+// cluster behind: 1 x 17344 9.8 / 11.8, 1 x 60656 18.7 / 32.3, 9x9 58x12x512 -> 4 14.9 / 24.9 (12560 10.2 / 10.3).
+constexpr int LONG_REDUCTION = 18000;
+enum class FewTiles { none, rows, gather, split, slices };
+static FewTiles few_tiles_form(Context &c, const ConvProblem &p)
 {
   if (c.opt_force_generic || c.opt_split_k != 0 || !igemm_tc_supported(c, p)) return FewTiles::none;
   const long long M = (long long)p.B * p.Ho * p.Wo;
@@ -436,6 +439,7 @@ static FewTiles few_tiles_form(const Context &c, const ConvProblem &p)
   const bool plain = p.ky * p.kx == 1 && p.H == p.Ho && p.W == p.Wo;
   bool few;
   const int tiles = igemm_tc_tiles(c, p, &few);
+  if (few && p.ky * p.kx * p.Cin >= LONG_REDUCTION && igemm_tc_slices(c, p) > 1) return FewTiles::slices;
   if (!plain) {
     if (tiles > sms || !few) return FewTiles::none;
     return (p.Cin % 128 == 0 && p.Cin >= 256) || !conv_gather_tc_supported(p) ? FewTiles::split : FewTiles::gather;
@@ -497,6 +501,7 @@ bool launch_conv(Context &c, const ConvProblem &p)
     case FewTiles::rows: return launch_gemm_fewrows(c, p);
     case FewTiles::gather: return launch_conv_gather_tc(c, p);
     case FewTiles::split: return launch_igemm_split(c, p);
+    case FewTiles::slices: return launch_igemm_tc(c, p, igemm_tc_slices(c, p));
     default: break;
   }
   // The SM-pair kernel: measured equal to the one-CTA kernel for K = 512 (0.054 against 0.053 ms on

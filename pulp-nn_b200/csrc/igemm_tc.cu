@@ -35,7 +35,7 @@
 //                      eight warps that alternate tiles, 256-column tiles by all sixteen.
 // All 512 columns of tensor memory are used as a ring of 512/BN accumulators, so the MMA issuers run
 // several tiles ahead of the epilogue. Integer accumulation is associative, so splitting K over
-// several CTAs (on request: PULPNN_OPT_SPLIT_K) gives bit-identical sums; partial sums then
+// several CTAs (longest reductions, or on request: PULPNN_OPT_SPLIT_K) gives bit-identical sums; partial sums then
 // go to a scratch buffer and a second kernel adds them and requantises. Rows of a short reduction
 // (K <= 64, N <= 64) are folded two or more to a GEMM row against a block-diagonal copy of W (see
 // launch_igemm_tc).
@@ -835,6 +835,17 @@ int igemm_tc_tiles(const Context &c, const ConvProblem &p, bool *few)
   return (int)(tiles < 0x7fffffff ? tiles : 0x7fffffff);
 }
 
+int igemm_tc_slices(Context &c, const ConvProblem &p)
+{
+  bool few;
+  const int sms = c.sm_count > 0 ? c.sm_count : 148, tiles = igemm_tc_tiles(c, p, &few), bkb = slab_bytes(p);
+  const int slabs = (p.ky * p.kx * p.Cin + bkb - 1) / bkb;
+  int slices = sms / tiles < slabs / 4 ? sms / tiles : slabs / 4;
+  if (slices > 16) slices = 16;
+  if (slices < 2) return 1;
+  return ctx_scratch_at_hand(c, (size_t)slices * p.B * p.Ho * p.Wo * p.Cout * sizeof(int)) ? slices : 1;
+}
+
 bool igemm_tc_few_values(const ConvProblem &p)
 {
   const long long rows = (long long)p.B * p.Ho * p.Wo;
@@ -852,7 +863,7 @@ double igemm_tc_spatial_estimate(const Context &c, const ConvProblem &p)
   return 2790 + rounds * (slabs * ((bkb == 128 ? 343 : (bkb == 64 ? 234 : 188)) + 0.0023 * bkb * (BM + bn)) + 5.3 * bn);
 }
 
-bool launch_igemm_tc(Context &c, const ConvProblem &p)
+bool launch_igemm_tc(Context &c, const ConvProblem &p, int slices)
 {
   TcParams g;
   g.M = p.B * p.Ho * p.Wo; g.N = p.Cout; g.K = p.ky * p.kx * p.Cin;
@@ -922,8 +933,7 @@ bool launch_igemm_tc(Context &c, const ConvProblem &p)
     bn = bn_try;
     g.n_tiles = (g.N + bn - 1) / bn;
     tiles = g.m_tiles * g.n_tiles;
-    // K is split here only on request: problems of few tiles and a long reduction go to igemm_split.cu
-    int slices = c.opt_split_k > 0 ? c.opt_split_k : 1;
+    if (c.opt_split_k > 0) slices = c.opt_split_k;
     if (slices > g.total_slabs) slices = g.total_slabs;
     if (slices < 1) slices = 1;
     g.slabs_per_slice = (g.total_slabs + slices - 1) / slices;

@@ -232,6 +232,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
 void *ctx_scratch(Context &c, size_t bytes);    // grow-only device scratch, nullptr on failure
+bool ctx_scratch_at_hand(Context &c, size_t bytes);     // false where that would allocate under a stream capture
 
 // A per-kernel setting that belongs to a device (cudaFuncSetAttribute, an occupancy figure) is
 // cached per device, not per process or per thread: one process may drive several GPUs, from one
@@ -280,7 +281,9 @@ bool conv_smallcin_supported(const ConvProblem &p);
 double conv_smallcin_estimate(const Context &c, const ConvProblem &p);        // ns of a problem it takes
 bool launch_conv_smallcin(Context &c, const ConvProblem &p);
 bool igemm_tc_supported(const Context &c, const ConvProblem &p);
-bool launch_igemm_tc(Context &c, const ConvProblem &p);
+bool launch_igemm_tc(Context &c, const ConvProblem &p, int slices = 1);   // K split over `slices` CTAs, sums through scratch
+// the slices for a long reduction of few tiles; 1 where their scratch cannot be had
+int igemm_tc_slices(Context &c, const ConvProblem &p);
 // whether its output rows are whole 16-byte pieces; otherwise it stores byte by byte
 bool igemm_tc_whole_rows(const Context &c, const ConvProblem &p);
 // whether a tile has so few values, behind so short a reduction, that storing them byte by byte does not matter

@@ -75,6 +75,54 @@ def test_first_layers(B, H, W, Cin, Cout, k, took, gpu, restatement):
     same(got[-1:], restatement.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
 
 
+# reductions on both sides of 18000 terms: a cluster, or slices whose sums go through memory, which under a stream
+# capture with no memory at hand go to the cluster
+@pytest.mark.parametrize("B,K,N,took", [(1, 17984, 20, "igemm_split_kernel"), (5, 18000, 20, "igemm_tc_kernel"), (130, 65520, 33, "igemm_tc_kernel")])
+def test_long_reductions(B, K, N, took, gpu, restatement):
+    c = wl.linear_case(134, K, N, batch=B, with_bias=True)
+    got = gpu.linear_out_32(c["x"], c["w"], bias32=c["bias32"])
+    assert api.last_kernel() == took
+    same(got, restatement.linear_out_32(c["x"], c["w"], bias32=c["bias32"]))
+    kw = dict(bias=c["bias"], out_mult=c["out_mult"], out_shift=14, relu=c["relu"], bn=c["bn"])
+    same(gpu.linear(32, c["x"], c["w"], c["k"], c["lam"], **kw), restatement.linear(32, c["x"], c["w"], c["k"], c["lam"], **kw))
+
+
+def test_long_convolution(gpu, restatement):
+    c = wl.conv_case(135, 9, 8, 448, 30, kernel=(7, 7), pads=(3, 3, 3, 3), out_shift=15)
+    got = gpu.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c))
+    assert api.last_kernel() == "igemm_tc_kernel"
+    same(got, restatement.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
+
+
+def test_long_reduction_first_under_capture(restatement):
+    import threading
+
+    import torch
+    c = wl.linear_case(136, 20000, 24, batch=3, with_bias=True)
+    put = lambda a: torch.from_numpy(a).cuda()  # noqa: E731
+    x, w, bias = put(c["x"]), put(c["w"]), put(c["bias32"])
+    out = torch.zeros((3, 24), dtype=torch.int32, device="cuda")
+    took = []
+
+    def work():                                  # a thread of its own has a context of its own, without scratch
+        torch.cuda.set_device(0)
+        api.set_device(0)
+        api.set_batch(3)
+        s, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            api.set_stream(s.cuda_stream)
+            api.pulp_nn_linear_out_32(32, x, bias, out, w, 20000, 24)
+        took.append(api.last_kernel())
+        g.replay()
+        torch.cuda.synchronize()
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert took == ["igemm_split_kernel"]
+    same(out.cpu().numpy(), restatement.linear_out_32(c["x"], c["w"], bias32=c["bias32"]))
+
+
 # depthwise layers with one row of output, of which the plane kernel computes two or four
 @pytest.mark.parametrize("B,W,C,k,s,hwc,took", [
     (1, 1958, 128, 3, 2, True, "depthwise_hwc3x3_tma_kernel"), (15, 80, 32, 3, 1, False, "depthwise_chw3x3_tma_kernel"),

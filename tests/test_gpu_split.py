@@ -42,7 +42,7 @@ def test_modes(bits, relu, bn, gpu, restatement):
 @pytest.mark.parametrize("batch,K,N", [(8, 1024, 16), (49, 1024, 1024), (128, 1024, 1000), (129, 4096, 33), (196, 512, 512),
                                        (200, 1168, 100), (256, 2048, 257), (300, 4096, 64), (5, 65520, 20), (300, 528, 48)])
 def test_linear(batch, K, N, gpu, restatement):
-    kernel = {8: "gemm_fewrows_kernel", 300: KERNEL if K > 1024 else "igemm_tc_kernel"}.get(batch, KERNEL)
+    kernel = {8: "gemm_fewrows_kernel", 5: "igemm_tc_kernel", 300: KERNEL if K > 1024 else "igemm_tc_kernel"}.get(batch, KERNEL)
     c = wl.linear_case(92, K, N, batch=batch, with_bias=True)
     got = gpu.linear_out_32(c["x"], c["w"], bias32=c["bias32"])
     assert api.last_kernel() == kernel
