@@ -485,14 +485,15 @@ bool launch_conv(Context &c, const ConvProblem &p)
     // A spatial kernel whose weights fit an SM: conv_halo_tc.cu, unless the estimates leave another kernel well ahead. Its
     // patches are 8x16 pixels whatever the image, its CTAs walk a long reduction alone: of one image row 3340 pixels long,
     // 3x1 288 -> 224 at batch 3, it makes 40.6 us against igemm_tc's 10.9; 3x3 11x4x416 -> 32, one image, 13.9 against
-    // 6.2 in the gathering kernel; 3x3 7x7x512 -> 512 9.9 against 7.1 in a cluster. Over 188 calls of odd sizes the choice
-    // is 1 % behind the fastest of the three kernels; always this one, 9 %.
+    // 6.2 in the gathering kernel; 3x3 7x7x512 -> 512 9.9 against 7.1 in a cluster. Over 1300 calls of odd sizes the
+    // choice is 2 to 3 % behind the fastest kernel of each, whatever the margin between 1.08 and 1.15; at 1.08 102x102x128 ->
+    // 128, one image with 64-bit parameters, went to igemm_tc: 9.2 against 7.9.
     const double halo = conv_halo_tc_estimate(c, p);
     if (halo >= 0) {
       const double gather = few == FewTiles::split ? -1 : conv_gather_tc_estimate(c, p);
       const double igemm = few == FewTiles::none ? igemm_tc_spatial_estimate(c, p) : -1;
       const double split = few == FewTiles::split ? igemm_split_estimate(c, p) : -1;
-      auto ahead = [&](double t, double u) { return t >= 0 && 1.08 * t < u; };
+      auto ahead = [&](double t, double u) { return t >= 0 && 1.15 * t < u; };
       if (!ahead(gather, halo) && !ahead(igemm, halo) && !ahead(split, halo)) return launch_conv_halo_tc(c, p);
       if (few == FewTiles::none) return gather >= 0 && gather < igemm ? launch_conv_gather_tc(c, p) : launch_igemm_tc(c, p);
     }

@@ -24,7 +24,7 @@ def _status():
     (3, 1, 3340, 288, 224, (1, 3), (1, 1), "igemm_tc_kernel"), (5, 1, 1201, 160, 32, (1, 3), (1, 1), "conv_gather_tc_kernel"),
     (30, 1, 2776, 32, 448, (1, 3), (1, 2), "igemm_tc_kernel"), (105, 4, 302, 416, 16, (3, 1), (1, 1), "conv_gather_tc_kernel"),
     (1, 11, 4, 416, 32, (3, 3), (1, 1), "conv_gather_tc_kernel"), (1, 4, 4, 96, 16, (9, 9), (2, 2), "conv_gather_tc_kernel"),
-    (1, 7, 7, 512, 512, (3, 3), (1, 1), "igemm_split_kernel"), (32, 28, 28, 128, 128, (3, 3), (1, 1), "conv_halo_tc_kernel")])
+    (1, 7, 7, 512, 512, (3, 3), (1, 1), "igemm_split_kernel"), (1, 102, 102, 128, 128, (3, 3), (1, 1), "conv_halo_tc_kernel"), (32, 28, 28, 128, 128, (3, 3), (1, 1), "conv_halo_tc_kernel")])
 def test_spatial_kernels(B, H, W, Cin, Cout, kernel, strides, took, gpu, restatement):
     c = wl.conv_case(130, H, W, Cin, Cout, kernel=kernel, strides=strides, pads=(kernel[0] // 2,) * 2 + (kernel[1] // 2,) * 2,
                      batch=B, out_shift=12)
