@@ -532,7 +532,8 @@ bool launch_conv_gather_tc(Context &c, const ConvProblem &p)
   g.by_last.set((unsigned)(p.Cout - (g.n_tiles - 1) * g.bn));
   g.by_cols.set((unsigned)(g.bn / 16));              // 16-byte pieces of a full tile's row
 
-  // two CTAs per SM: the ring (at least three stages, which also hold the output tile) and, if it fits, all of W
+  // two CTAs per SM: the ring, which also holds the output tile, and, if it fits beside three stages, all of W (two
+  // stages where 256 columns of W are streamed)
   const int half_sm = SMEM_SM / 2 - STATIC_SMEM - SMEM_RESERVED - 1024;
   const long long w_all = (long long)g.slabs_per * g.bn * 128;
   const bool w_res = w_all + 3 * A_STAGE <= half_sm;

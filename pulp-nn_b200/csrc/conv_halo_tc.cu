@@ -16,8 +16,8 @@
 // What bounds it: the MMAs -- one costs some 80 cycles, bound by reading 32 bytes of each of its rows, so the issuing
 // thread adds a tabled offset per tap and nothing else (with the offsets computed there a tap of one MMA took 270
 // cycles) --, for 32- and 64-channel slabs the rows of the TMA box, and a last round of tiles that is not full.
-// Measured (us, graph replay, the kernel before / this one): 3x3 28x28x128 -> 128 at batch 32 11.9 / 8.1, at batch 1 6.7 /
-// 5.1; 56x56x64 -> 64 at batch 64 31.3 / 20.1; 112x112x64 -> 64 at batch 16 31.4 / 17.8; 56x56x96 -> 96 at batch 32
+// Measured (us, graph replay, the kernel before / this one): 3x3 28x28x128 -> 128 at batch 32 11.9 / 8.3, at batch 1 6.7 /
+// 4.6; 56x56x64 -> 64 at batch 64 31.3 / 20.1; 112x112x64 -> 64 at batch 16 31.4 / 17.8; 56x56x96 -> 96 at batch 32
 // 27.8 / 20.6; 32x32x32 -> 64 at batch 1 4.5 / 3.4; 5x5 28x28x64 -> 64 at batch 32 17.0 / 9.0; stride 2 56x56x64 -> 128 at
 // batch 32 8.8 / 6.9. Tried: a staging tile and 16-byte pieces instead of 32-byte stores, with 8 warps: 8.0 and 22.3
 // us on the first two (before the issue loop was cut down; with four groups of epilogue warps 8.8 and 23.3).

@@ -425,8 +425,9 @@ void add_entry(uint8_t *a, uint8_t *b, uint8_t *out, int m1, int m2, int out_shi
 //   1 x 1024 -> 1000     8.2 / 5.2 / 4.9,  2.2      37 x 1024 -> 1000  9.2 / 5.6 / 5.1,  4.8     128 x 1024 -> 1000  13.2 / 5.8 / 5.2, 11.8
 //   1 x 4096 -> 4096     9.9 / 18  / 9.4,  5.6      16 x 4096 -> 4096  10.4 / 19 / 9.8, 13.9     128 x 4096 -> 4096  16.5 / 20 / 10.3, 87
 //   256 x 4096 -> 4096  17.4 / 33  / 13.0           512 x 4096 -> 4096 17.5 / 34 / 19.4          784 x 1024 -> 1024  7.7 / 9.8 / 9.2
-//   3x3, one image: 32x32x32 -> 64 8.1 / 4.4 / 7.7, 14x14x64 -> 64 8.1 / 5.4 / 7.5, 28x28x128 -> 128 10.4 / 6.6 / 6.8,
-//   7x7x512 -> 512 10.1 / 8.5 / 7.1; 14x14x256 -> 256 at batch 8 14.3 / 11.1 / 9.1, 28x28x128 -> 128 at batch 4 7.4 / 9.1 / 8.2
+//   3x3, one image: 7x7x512 -> 512 10.1 / 8.5 / 7.1; of shapes that conv_halo_tc takes first today (its time last): 32x32x32
+//   -> 64 8.1 / 4.4 / 7.7 / 3.5, 14x14x64 -> 64 8.1 / 5.4 / 7.5 / 3.9, 28x28x128 -> 128 10.4 / 6.6 / 6.8 / 4.6, at batch 4
+//   7.4 / 9.1 / 8.2 / 5.3, 14x14x256 -> 256 at batch 8 14.3 / 11.1 / 9.1 / 7.2
 // Beyond 18000 terms the 16 slices of a split through memory (igemm_tc and a second kernel) leave the eight CTAs of a
 // cluster behind: 1 x 17344 9.8 / 11.8, 1 x 60656 18.7 / 32.3, 9x9 58x12x512 -> 4 14.9 / 24.9 (12560 10.2 / 10.3).
 constexpr int LONG_REDUCTION = 18000;
@@ -463,11 +464,11 @@ static FewTiles few_tiles_form(Context &c, const ConvProblem &p)
 // 32 78 / 12, 18x18x32 -> 77 at batch 59 19.6 / 6.6, 3x3 28x28x64 -> 100 at batch 16 19.7 / 8.6 (equal only for 3x3
 // 14x14x256 -> 77: 20.6 / 21.6) -- unless these are few: igemm_tc has the shorter start (24 vectors of 48 -> 3 2.8 / 4.8,
 // 128 -> 2 over 97x97 pixels 3.2 / 3.8; of 173 such calls of up to 1700 values a tile and five slabs, 7 are better off in
-// the gathering kernel; beyond 2200 values or eight slabs the lines cross). Spatial kernels on channel slabs of 32 bytes, up to 192 output channels: 56x56x96 -> 96
-// at batch 32 43.9 / 27.4, 28x28x160 -> 160 24.9 / 18.8, 56x56x32 -> 64 at batch 64 29.5 / 22.6, 28x28x32 -> 128 11.7 /
-// 11.8; 32 -> 256 13.3 / 16.9, 224 -> 224 18.4 / 19.4. Slabs of 64 bytes, up to 64 channels and enough tiles: 56x56x64
-// -> 64 at batch 64 36.4 / 30.8, at batch 16 13.0 / 12.5; one image 5.3 / 6.7. (The spatial kernels whose weights fit an
-// SM do not come here: conv_halo_tc.cu takes them first.)
+// the gathering kernel; beyond 2200 values or eight slabs the lines cross). Spatial kernels on channel slabs of 32 bytes,
+// up to 192 output channels: 3x3 224 -> 224 over 28x28 at batch 16 18.4 / 19.4; slabs of 64 bytes, up to 64 channels and
+// enough tiles. Most of these conv_halo_tc takes first; the lines were drawn before it, on (its time last) 56x56x96 -> 96 at
+// batch 32 43.9 / 27.4 / 20.5, 28x28x160 -> 160 24.9 / 18.8 / 19.3, 56x56x32 -> 64 at batch 64 29.5 / 22.6 / 16.4, 56x56x64
+// -> 64 at batch 64 36.4 / 30.8 / 20.5, and hold for what it leaves.
 static bool gather_first(const Context &c, const ConvProblem &p)
 {
   if (c.opt_split_k != 0 || !conv_gather_tc_supported(p)) return false;
