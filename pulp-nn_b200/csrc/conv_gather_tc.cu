@@ -507,9 +507,13 @@ static bool gather_aligned(const ConvProblem &p)
 
 // Fitted to 1900 calls of 2 to 300 us (standard deviation 11 %): a tile's slabs by the rows gathered for each, twice as
 // dear where chunks cross pixels, its drain by the columns, and the exchange of a shared reduction.
-double conv_gather_tc_estimate(const Context &c, const ConvProblem &p)
+double conv_gather_tc_estimate(const Context &c, const ConvProblem &p, double worth)
 {
   if (!conv_gather_tc_supported(p)) return -1;
+  // one round of the smallest tiles over an eighth of the slabs: the plan is looked for only if that is of interest
+  const int eighth = ((p.ky * ((p.kx * p.Cin + 15) / 16) + 7) / 8 + 7) / 8;
+  const double least = 2960 + (gather_aligned(p) ? 4.7 : 8.3) * eighth * (GBM + 16);
+  if (least >= worth) return least;
   GatherParams g = {};
   const double rounds = (double)plan_gather(p, c.sm_count > 0 ? c.sm_count : 148, g);
   return 2060 + rounds * (900 + (gather_aligned(p) ? 4.7 : 8.3) * g.slabs_per * (GBM + g.bn) + 10 * g.bn) + (g.k_split > 1 ? 46 * g.bn : 0);

@@ -491,7 +491,7 @@ bool launch_conv(Context &c, const ConvProblem &p)
     // 128, one image with 64-bit parameters, went to igemm_tc: 9.2 against 7.9.
     const double halo = conv_halo_tc_estimate(c, p);
     if (halo >= 0) {
-      const double gather = few == FewTiles::split ? -1 : conv_gather_tc_estimate(c, p);
+      const double gather = few == FewTiles::split ? -1 : conv_gather_tc_estimate(c, p, halo / 1.15);
       const double igemm = few == FewTiles::none ? igemm_tc_spatial_estimate(c, p) : -1;
       const double split = few == FewTiles::split ? igemm_split_estimate(c, p) : -1;
       auto ahead = [&](double t, double u) { return t >= 0 && 1.15 * t < u; };
@@ -519,8 +519,8 @@ bool launch_conv(Context &c, const ConvProblem &p)
   // -> 32 channels 3.4 / 4.9, 21 of 575x291x1 -> 16 130 / 210, 64 of 28x28x1 -> 16 4.5 / 6.9; 16 of 28x28x1, 5x5, 5.7 / 4.7,
   // 16 of 96x96x3 -> 24 77 / 13). Over 500 calls the estimates are 1 % behind the faster of the two, by 5 % in 33 of them.
   if (!c.opt_force_generic && conv_smallcin_supported(p)) {
-    const double gather = conv_gather_tc_estimate(c, p);
-    if (gather < 0 || conv_smallcin_estimate(c, p) < gather) return launch_conv_smallcin(c, p);
+    const double strips = conv_smallcin_estimate(c, p), gather = conv_gather_tc_estimate(c, p, strips);
+    if (gather < 0 || strips < gather) return launch_conv_smallcin(c, p);
   }
   // 32-bit outputs of a reduction of at most 44 terms: the dp4a kernel starts sooner and stores its words as they are (2
   // vectors of 4 -> 4 2.8 us against 4.9, 58 of 8 -> 1896 4.0 / 5.4; of 30 such calls two, of 35 and 41 terms over 900

@@ -273,7 +273,8 @@ double conv_halo_tc_estimate(const Context &c, const ConvProblem &p);
 bool launch_conv_halo_tc(Context &c, const ConvProblem &p);
 // any channel count and alignment on the tensor cores, the im2col rows gathered by the warps
 bool conv_gather_tc_supported(const ConvProblem &p);
-double conv_gather_tc_estimate(const Context &c, const ConvProblem &p);       // ns, -1 where it does not take the problem
+// ns, or a lower bound that is not below `worth`; -1 where it does not take the problem
+double conv_gather_tc_estimate(const Context &c, const ConvProblem &p, double worth);
 bool launch_conv_gather_tc(Context &c, const ConvProblem &p);
 bool conv_smallcin_tc_supported(const ConvProblem &p);
 bool launch_conv_smallcin_tc(Context &c, const ConvProblem &p);
