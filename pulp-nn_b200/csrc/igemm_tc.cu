@@ -47,6 +47,8 @@
 #include <cstdio>
 #include <mutex>
 
+#include <type_traits>
+
 #include "internal.cuh"
 #include "sm100_primitives.cuh"
 #include "tensor_maps.cuh"
@@ -426,6 +428,39 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     long long *p_l64 = p_k64 + HALF_COLS;
     int staged_nt = -1;
     bool fits = false;                                             // EPI_BN64: 32-bit arithmetic gives the same (internal.cuh)
+    // 32 accumulator columns, parameter slots lc on, -> 32 bytes. The two arithmetics of 64-bit batch norm are loops of their
+    // own: with the choice inside one loop the 64-bit one took 5 % longer (14x14x512 -> 512 at batch 512 38.7 us, 40.7
+    // with it, 39.1 apart)
+    auto requant32 = [&](auto narrow, const uint32_t (&v)[32], int lc, unsigned (&w)[8]) {
+      if constexpr (MODE == EPI_BN32 || decltype(narrow)::value) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          const int4 kk = *reinterpret_cast<const int4 *>(p_k32 + lc + j);
+          const int4 ll = *reinterpret_cast<const int4 *>(p_l32 + lc + j);
+          w[j >> 2] = pack4_sat_u8((int)((unsigned)kk.x * v[j + 0] + (unsigned)ll.x) >> e.shift,
+                                   (int)((unsigned)kk.y * v[j + 1] + (unsigned)ll.y) >> e.shift,
+                                   (int)((unsigned)kk.z * v[j + 2] + (unsigned)ll.z) >> e.shift,
+                                   (int)((unsigned)kk.w * v[j + 3] + (unsigned)ll.w) >> e.shift);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          int q[4];
+#pragma unroll
+          for (int t = 0; t < 4; t++) {
+            const int a = (int)v[j + t];
+            if (MODE == EPI_BN64)
+              q[t] = (int)((long long)((unsigned long long)p_k64[lc + j + t] * (unsigned long long)(long long)a +
+                                       (unsigned long long)p_l64[lc + j + t]) >> e.shift);
+            else if (MODE == EPI_MULT)
+              q[t] = (int)(short)((int)((unsigned)e.out_mult * (unsigned)(a + p_bias[lc + j + t])) >> e.shift);
+            else
+              q[t] = (a + p_bias[lc + j + t]) >> e.shift;
+          }
+          w[j >> 2] = pack4_sat_u8(q[0], q[1], q[2], q[3]);
+        }
+      }
+    };
     // TMA_OUT: the group's staging tile, and the one thread of the group that issues its stores
     uint8_t *out_tile = smem + L::OUT_OFFSET + grp * L::OUT_TILE_BYTES;
     const bool elected = ((warp - FIRST_EPI) % (4 * NSPLIT)) == 0 && lane == 0;
@@ -506,38 +541,19 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
         for (int rd = 0; rd < ROUNDS; rd++) {
           if (!dead) {
+            auto chunks = [&](auto narrow) {
 #pragma unroll
-            for (int cr = 0; cr < CPR; cr++) {
-              const int ch = rd * CPR + cr;
-              const int lc = ch * 32, c0 = ch * (32 * NSPLIT) + half * 32;
-              uint32_t v[32];
-              tmem_ld_32(t_row + (uint32_t)c0, v);
-              tmem_wait_ld();
-#pragma unroll
-              for (int j = 0; j < 32; j += 4) {
-                int q[4];
-                if (MODE == EPI_BN32 || (MODE == EPI_BN64 && fits)) {
-                  const int4 kk = *reinterpret_cast<const int4 *>(p_k32 + lc + j);
-                  const int4 ll = *reinterpret_cast<const int4 *>(p_l32 + lc + j);
-                  q[0] = (int)((unsigned)kk.x * v[j + 0] + (unsigned)ll.x) >> e.shift;
-                  q[1] = (int)((unsigned)kk.y * v[j + 1] + (unsigned)ll.y) >> e.shift;
-                  q[2] = (int)((unsigned)kk.z * v[j + 2] + (unsigned)ll.z) >> e.shift;
-                  q[3] = (int)((unsigned)kk.w * v[j + 3] + (unsigned)ll.w) >> e.shift;
-                } else if (MODE == EPI_BN64) {
-                  requant4_bn64(p_k64 + lc + j, p_l64 + lc + j, v[j], v[j + 1], v[j + 2], v[j + 3], e.shift, false, q);
-                } else {
-#pragma unroll
-                  for (int t = 0; t < 4; t++) {
-                    const int a = (int)v[j + t];
-                    if (MODE == EPI_MULT)
-                      q[t] = (int)(short)((int)((unsigned)e.out_mult * (unsigned)(a + p_bias[lc + j + t])) >> e.shift);
-                    else
-                      q[t] = (a + p_bias[lc + j + t]) >> e.shift;
-                  }
-                }
-                w[ch][j >> 2] = pack4_sat_u8(q[0], q[1], q[2], q[3]);
+              for (int cr = 0; cr < CPR; cr++) {
+                const int ch = rd * CPR + cr;
+                const int lc = ch * 32, c0 = ch * (32 * NSPLIT) + half * 32;
+                uint32_t v[32];
+                tmem_ld_32(t_row + (uint32_t)c0, v);
+                tmem_wait_ld();
+                requant32(narrow, v, lc, w[ch]);
               }
-            }
+            };
+            if (MODE == EPI_BN64 && fits) chunks(std::bool_constant<MODE == EPI_BN64>{});
+            else chunks(std::false_type{});
             if (rd == ROUNDS - 1) {
               // the accumulator is in registers: hand it back to the MMA warps before the stores
               tc_fence_before();
@@ -597,81 +613,62 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         m = (cb * g.Ho + cy) * g.Wo + cx;
       }
       const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * BN_TILE);
+      auto chunks = [&](auto narrow) {
 #pragma unroll 1
-      for (int lc = 0; lc < HALF_COLS; lc += 32) {   // lc: offset inside this warp's parameter copy
-        const int c0 = (lc >> 5) * (32 * NSPLIT) + half * 32;   // column offset inside the tile
-        if (n0 + c0 >= g.N) break;                   // uniform across the warp
-        uint32_t v[32];
-        tmem_ld_32(t_row + (uint32_t)c0, v);
-        tmem_wait_ld();
-        if (PARTIAL || MODE == EPI_RAW32) {
-          int *orow = reinterpret_cast<int *>(g.out) +
-                      ((size_t)(PARTIAL ? ks : 0) * g.M + (size_t)(row_ok ? m : 0)) * g.N + n0 + c0;
-          if (row_ok) {
-            if (g.vec_store) {
+        for (int lc = 0; lc < HALF_COLS; lc += 32) {   // lc: offset inside this warp's parameter copy
+          const int c0 = (lc >> 5) * (32 * NSPLIT) + half * 32;   // column offset inside the tile
+          if (n0 + c0 >= g.N) break;                   // uniform across the warp
+          uint32_t v[32];
+          tmem_ld_32(t_row + (uint32_t)c0, v);
+          tmem_wait_ld();
+          if (PARTIAL || MODE == EPI_RAW32) {
+            int *orow = reinterpret_cast<int *>(g.out) +
+                        ((size_t)(PARTIAL ? ks : 0) * g.M + (size_t)(row_ok ? m : 0)) * g.N + n0 + c0;
+            if (row_ok) {
+              if (g.vec_store) {
 #pragma unroll
-              for (int i = 0; i < 32; i += 4) {
-                if (n0 + c0 + i < g.N) {
-                  int4 o;
-                  o.x = (int)v[i]; o.y = (int)v[i + 1]; o.z = (int)v[i + 2]; o.w = (int)v[i + 3];
-                  if (!PARTIAL) {
-                    const int4 bb = *reinterpret_cast<const int4 *>(p_bias + lc + i);
-                    o.x += bb.x; o.y += bb.y; o.z += bb.z; o.w += bb.w;
+                for (int i = 0; i < 32; i += 4) {
+                  if (n0 + c0 + i < g.N) {
+                    int4 o;
+                    o.x = (int)v[i]; o.y = (int)v[i + 1]; o.z = (int)v[i + 2]; o.w = (int)v[i + 3];
+                    if (!PARTIAL) {
+                      const int4 bb = *reinterpret_cast<const int4 *>(p_bias + lc + i);
+                      o.x += bb.x; o.y += bb.y; o.z += bb.z; o.w += bb.w;
+                    }
+                    *reinterpret_cast<int4 *>(orow + i) = o;
                   }
-                  *reinterpret_cast<int4 *>(orow + i) = o;
                 }
-              }
-            } else {
+              } else {
 #pragma unroll
-              for (int i = 0; i < 32; i++)
-                if (n0 + c0 + i < g.N) orow[i] = (int)v[i] + (PARTIAL ? 0 : p_bias[lc + i]);
-            }
-          }
-        } else {
-          unsigned w[8];
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            int q[4];
-            if (MODE == EPI_BN32 || (MODE == EPI_BN64 && fits)) {
-              const int4 kk = *reinterpret_cast<const int4 *>(p_k32 + lc + i);
-              const int4 ll = *reinterpret_cast<const int4 *>(p_l32 + lc + i);
-              q[0] = (int)((unsigned)kk.x * v[i + 0] + (unsigned)ll.x) >> e.shift;
-              q[1] = (int)((unsigned)kk.y * v[i + 1] + (unsigned)ll.y) >> e.shift;
-              q[2] = (int)((unsigned)kk.z * v[i + 2] + (unsigned)ll.z) >> e.shift;
-              q[3] = (int)((unsigned)kk.w * v[i + 3] + (unsigned)ll.w) >> e.shift;
-            } else if (MODE == EPI_BN64) {
-              requant4_bn64(p_k64 + lc + i, p_l64 + lc + i, v[i], v[i + 1], v[i + 2], v[i + 3], e.shift, false, q);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 4; j++) {
-                const int a = (int)v[i + j];
-                if (MODE == EPI_MULT)
-                  q[j] = (int)(short)((int)((unsigned)e.out_mult * (unsigned)(a + p_bias[lc + i + j])) >> e.shift);
-                else
-                  q[j] = (a + p_bias[lc + i + j]) >> e.shift;
+                for (int i = 0; i < 32; i++)
+                  if (n0 + c0 + i < g.N) orow[i] = (int)v[i] + (PARTIAL ? 0 : p_bias[lc + i]);
               }
             }
-            w[i >> 2] = pack4_sat_u8(q[0], q[1], q[2], q[3]);
-          }
-          if (row_ok) {
-            uint8_t *orow = reinterpret_cast<uint8_t *>(g.out) + (size_t)m * g.N + n0 + c0;
-            if (g.vec_store == 2) {
-              // one full 32-byte sector per lane and instruction
-              asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                           ::"l"(orow), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]),
-                             "r"(w[6]), "r"(w[7])
-                           : "memory");
-            } else if (g.vec_store == 1) {
-              if (n0 + c0 < g.N) *reinterpret_cast<uint4 *>(orow) = make_uint4(w[0], w[1], w[2], w[3]);
-              if (n0 + c0 + 16 < g.N) *reinterpret_cast<uint4 *>(orow + 16) = make_uint4(w[4], w[5], w[6], w[7]);
-            } else {
+          } else {
+            unsigned w[8];
+            requant32(narrow, v, lc, w);
+            if (row_ok) {
+              uint8_t *orow = reinterpret_cast<uint8_t *>(g.out) + (size_t)m * g.N + n0 + c0;
+              if (g.vec_store == 2) {
+                // one full 32-byte sector per lane and instruction
+                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                             ::"l"(orow), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]),
+                               "r"(w[6]), "r"(w[7])
+                             : "memory");
+              } else if (g.vec_store == 1) {
+                if (n0 + c0 < g.N) *reinterpret_cast<uint4 *>(orow) = make_uint4(w[0], w[1], w[2], w[3]);
+                if (n0 + c0 + 16 < g.N) *reinterpret_cast<uint4 *>(orow + 16) = make_uint4(w[4], w[5], w[6], w[7]);
+              } else {
 #pragma unroll
-              for (int i = 0; i < 32; i++)
-                if (n0 + c0 + i < g.N) orow[i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
+                for (int i = 0; i < 32; i++)
+                  if (n0 + c0 + i < g.N) orow[i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
+              }
             }
           }
         }
-      }
+      };
+      if (MODE == EPI_BN64 && fits) chunks(std::bool_constant<MODE == EPI_BN64>{});
+      else chunks(std::false_type{});
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[acc]);
