@@ -101,12 +101,32 @@ void *ctx_scratch(Context &c, size_t bytes)
   return c.scratch;
 }
 
-bool ctx_scratch_at_hand(Context &c, size_t bytes)
+// Not under a stream capture: a graph would keep the address while the buffer grows, and be replayed on any stream.
+void *ctx_partials(Context &c, size_t bytes)
 {
-  if (bytes <= c.scratch_cap) return true;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(c.stream, &cap) != cudaSuccess) { cudaGetLastError(); return false; }
-  return cap == cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c.stream, &cap) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  if (cap != cudaStreamCaptureStatusNone) return nullptr;
+  if (!c.partials_done && cudaEventCreateWithFlags(&c.partials_done, cudaEventDisableTiming) != cudaSuccess) {
+    cudaGetLastError();
+    c.partials_done = nullptr;
+    return nullptr;
+  }
+  if (bytes > c.partials_cap) {
+    cudaEventSynchronize(c.partials_done);
+    if (c.partials) cudaFree(c.partials);
+    c.partials = nullptr; c.partials_cap = 0;
+    const size_t size = (bytes + (1u << 20) - 1) & ~(size_t)((1u << 20) - 1);
+    if (cudaMalloc(&c.partials, size) != cudaSuccess) { cudaGetLastError(); c.partials = nullptr; return nullptr; }
+    c.partials_cap = size;
+  }
+  if (cudaStreamWaitEvent(c.stream, c.partials_done, 0) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  return c.partials;
+}
+
+bool ctx_partials_done(Context &c)
+{
+  return cuda_ok(cudaEventRecord(c.partials_done, c.stream), "cudaEventRecord(partial sums)");
 }
 
 // device word that kernels with bounded waits report into (read by pulpnn_device_status)
@@ -206,6 +226,10 @@ int pulpnn_set_device(int device)
     for (auto &s : c.slots) { if (s.dev) cudaFree(s.dev); s.dev = nullptr; s.cap = 0; }
     if (c.scratch) cudaFree(c.scratch);
     c.scratch = nullptr; c.scratch_cap = 0;
+    if (c.partials) cudaFree(c.partials);
+    c.partials = nullptr; c.partials_cap = 0;
+    if (c.partials_done) cudaEventDestroy(c.partials_done);
+    c.partials_done = nullptr;
     if (c.status_word) cudaFree(c.status_word);
     c.status_word = nullptr;
     c.device = -1;

@@ -429,7 +429,7 @@ void add_entry(uint8_t *a, uint8_t *b, uint8_t *out, int m1, int m2, int out_shi
 //   -> 64 8.1 / 4.4 / 7.7 / 3.5, 14x14x64 -> 64 8.1 / 5.4 / 7.5 / 3.9, 28x28x128 -> 128 10.4 / 6.6 / 6.8 / 4.6, at batch 4
 //   7.4 / 9.1 / 8.2 / 5.3, 14x14x256 -> 256 at batch 8 14.3 / 11.1 / 9.1 / 7.2
 // Beyond 18000 terms the 16 slices of a split through memory (igemm_tc and a second kernel) leave the eight CTAs of a
-// cluster behind: 1 x 17344 9.8 / 11.8, 1 x 60656 18.7 / 32.3, 9x9 58x12x512 -> 4 14.9 / 24.9 (12560 10.2 / 10.3).
+// cluster behind (not under a stream capture, whose graph would keep that memory's address): 1 x 17344 9.8 / 11.8, 1 x 60656 18.7 / 32.3, 9x9 58x12x512 -> 4 14.9 / 24.9 (12560 10.2 / 10.3).
 constexpr int LONG_REDUCTION = 18000;
 enum class FewTiles { none, rows, gather, split, slices };
 static FewTiles few_tiles_form(Context &c, const ConvProblem &p)
@@ -440,7 +440,10 @@ static FewTiles few_tiles_form(Context &c, const ConvProblem &p)
   const bool plain = p.ky * p.kx == 1 && p.H == p.Ho && p.W == p.Wo;
   bool few;
   const int tiles = igemm_tc_tiles(c, p, &few);
-  if (few && p.ky * p.kx * p.Cin >= LONG_REDUCTION && igemm_tc_slices(c, p) > 1) return FewTiles::slices;
+  if (few && p.ky * p.kx * p.Cin >= LONG_REDUCTION) {
+    const int slices = igemm_tc_slices(c, p);
+    if (slices > 1 && igemm_tc_partials(c, p, slices)) return FewTiles::slices;
+  }
   if (!plain) {
     if (tiles > sms || !few) return FewTiles::none;
     return (p.Cin % 128 == 0 && p.Cin >= 256) || !conv_gather_tc_supported(p) ? FewTiles::split : FewTiles::gather;

@@ -832,15 +832,18 @@ int igemm_tc_tiles(const Context &c, const ConvProblem &p, bool *few)
   return (int)(tiles < 0x7fffffff ? tiles : 0x7fffffff);
 }
 
-int igemm_tc_slices(Context &c, const ConvProblem &p)
+int igemm_tc_slices(const Context &c, const ConvProblem &p)
 {
   bool few;
   const int sms = c.sm_count > 0 ? c.sm_count : 148, tiles = igemm_tc_tiles(c, p, &few), bkb = slab_bytes(p);
   const int slabs = (p.ky * p.kx * p.Cin + bkb - 1) / bkb;
   int slices = sms / tiles < slabs / 4 ? sms / tiles : slabs / 4;
-  if (slices > 16) slices = 16;
-  if (slices < 2) return 1;
-  return ctx_scratch_at_hand(c, (size_t)slices * p.B * p.Ho * p.Wo * p.Cout * sizeof(int)) ? slices : 1;
+  return slices < 2 ? 1 : (slices > 16 ? 16 : slices);
+}
+
+bool igemm_tc_partials(Context &c, const ConvProblem &p, int slices)
+{
+  return ctx_partials(c, (size_t)slices * p.B * p.Ho * p.Wo * p.Cout * sizeof(int)) != nullptr;
 }
 
 bool igemm_tc_few_values(const ConvProblem &p)
@@ -924,13 +927,14 @@ bool launch_igemm_tc(Context &c, const ConvProblem &p, int slices)
   // uint8 tiles can leave through TMA stores (staged in shared memory, at most 128 columns wide)
   const bool out_ok = !raw && g.N % 16 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
 
+  const bool requested = c.opt_split_k > 0;          // PULPNN_OPT_SPLIT_K
   int bn = 0, tiles = 0;
   bool tma_out = false;
   auto configure = [&](int bn_try, bool tma_try) {
     bn = bn_try;
     g.n_tiles = (g.N + bn - 1) / bn;
     tiles = g.m_tiles * g.n_tiles;
-    if (c.opt_split_k > 0) slices = c.opt_split_k;
+    if (requested) slices = c.opt_split_k;
     if (slices > g.total_slabs) slices = g.total_slabs;
     if (slices < 1) slices = 1;
     g.slabs_per_slice = (g.total_slabs + slices - 1) / slices;
@@ -993,7 +997,7 @@ bool launch_igemm_tc(Context &c, const ConvProblem &p, int slices)
     return launch_final(c, maps, g, bn, bkb, grid, tma_out);
   }
   const size_t part_bytes = (size_t)g.k_slices * g.M * g.N * sizeof(int);
-  int *partials = static_cast<int *>(ctx_scratch(c, part_bytes));
+  int *partials = static_cast<int *>(requested ? ctx_scratch(c, part_bytes) : c.partials);
   if (!partials) return false;
   g.out = partials;
   g.vec_store = (g.N % 4 == 0);
@@ -1009,7 +1013,8 @@ bool launch_igemm_tc(Context &c, const ConvProblem &p, int slices)
     default:       splitk_reduce_kernel<EPI_RAW32><<<blocks, 256, 0, c.stream>>>(partials, p.out, p.epi, g.M, g.N, g.k_slices); break;
   }
   count_launch();
-  return cuda_ok(cudaGetLastError(), "splitk_reduce launch");
+  const bool ok = cuda_ok(cudaGetLastError(), "splitk_reduce launch");
+  return (requested || ctx_partials_done(c)) && ok;
 }
 
 #ifdef PULPNN_TRACE

@@ -196,6 +196,9 @@ struct Context {
   StageSlot slots[8];
   // device scratch owned by the context (split-K partial sums, status word)
   void *scratch = nullptr; size_t scratch_cap = 0;
+  // partial sums of the longest reductions, and when their latest reader was through with them
+  void *partials = nullptr; size_t partials_cap = 0;
+  cudaEvent_t partials_done = nullptr;
   int *status_word = nullptr;     // device int, 0 = fine
   int sm_count = 0;
 };
@@ -232,7 +235,10 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
 void *ctx_scratch(Context &c, size_t bytes);    // grow-only device scratch, nullptr on failure
-bool ctx_scratch_at_hand(Context &c, size_t bytes);     // false where that would allocate under a stream capture
+// Memory for partial sums that the context's stream may write from now on, whichever stream used it before; nullptr, and
+// no error, under a stream capture and where there is none to be had. ctx_partials_done() after the last kernel that reads them.
+void *ctx_partials(Context &c, size_t bytes);
+bool ctx_partials_done(Context &c);
 
 // A per-kernel setting that belongs to a device (cudaFuncSetAttribute, an occupancy figure) is
 // cached per device, not per process or per thread: one process may drive several GPUs, from one
@@ -282,9 +288,10 @@ bool conv_smallcin_supported(const ConvProblem &p);
 double conv_smallcin_estimate(const Context &c, const ConvProblem &p);        // ns of a problem it takes
 bool launch_conv_smallcin(Context &c, const ConvProblem &p);
 bool igemm_tc_supported(const Context &c, const ConvProblem &p);
-bool launch_igemm_tc(Context &c, const ConvProblem &p, int slices = 1);   // K split over `slices` CTAs, sums through scratch
-// the slices for a long reduction of few tiles; 1 where their scratch cannot be had
-int igemm_tc_slices(Context &c, const ConvProblem &p);
+// `slices`: K split over so many CTAs, whose sums go through memory that igemm_tc_partials() got just before
+bool launch_igemm_tc(Context &c, const ConvProblem &p, int slices = 1);
+int igemm_tc_slices(const Context &c, const ConvProblem &p);    // for a long reduction of few tiles
+bool igemm_tc_partials(Context &c, const ConvProblem &p, int slices);     // false (no error) where there is none to be had
 // whether its output rows are whole 16-byte pieces; otherwise it stores byte by byte
 bool igemm_tc_whole_rows(const Context &c, const ConvProblem &p);
 // whether a tile has so few values, behind so short a reduction, that storing them byte by byte does not matter

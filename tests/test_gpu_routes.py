@@ -75,8 +75,8 @@ def test_first_layers(B, H, W, Cin, Cout, k, took, gpu, restatement):
     same(got[-1:], restatement.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
 
 
-# reductions on both sides of 18000 terms: a cluster, or slices whose sums go through memory, which under a stream
-# capture with no memory at hand go to the cluster
+# reductions on both sides of 18000 terms: a cluster, or slices whose sums go through memory, which a stream capture may not
+# hold on to and two streams of a thread share
 @pytest.mark.parametrize("B,K,N,took", [(1, 17984, 20, "igemm_split_kernel"), (5, 18000, 20, "igemm_tc_kernel"), (130, 65520, 33, "igemm_tc_kernel")])
 def test_long_reductions(B, K, N, took, gpu, restatement):
     c = wl.linear_case(134, K, N, batch=B, with_bias=True)
@@ -94,7 +94,8 @@ def test_long_convolution(gpu, restatement):
     same(got, restatement.conv(32, c["x"], c["w"], c["k"], c["lam"], **conv_kw(c)))
 
 
-def test_long_reduction_first_under_capture(restatement):
+@pytest.mark.parametrize("first", ["eager", "captured"])
+def test_long_reduction_under_capture(first, restatement):
     import threading
 
     import torch
@@ -104,11 +105,16 @@ def test_long_reduction_first_under_capture(restatement):
     out = torch.zeros((3, 24), dtype=torch.int32, device="cuda")
     took = []
 
-    def work():                                  # a thread of its own has a context of its own, without scratch
+    def work():                                  # a thread of its own has a context of its own, without memory for sums
         torch.cuda.set_device(0)
         api.set_device(0)
         api.set_batch(3)
         s, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        if first == "eager":
+            api.pulp_nn_linear_out_32(32, x, bias, out, w, 20000, 24)
+            took.append(api.last_kernel())
+            torch.cuda.synchronize()
+            out.zero_()
         with torch.cuda.graph(g, stream=s):
             api.set_stream(s.cuda_stream)
             api.pulp_nn_linear_out_32(32, x, bias, out, w, 20000, 24)
@@ -119,8 +125,33 @@ def test_long_reduction_first_under_capture(restatement):
     t = threading.Thread(target=work)
     t.start()
     t.join()
-    assert took == ["igemm_split_kernel"]
+    assert took == ["igemm_tc_kernel"] * (first == "eager") + ["igemm_split_kernel"]
     same(out.cpu().numpy(), restatement.linear_out_32(c["x"], c["w"], bias32=c["bias32"]))
+
+
+def test_long_reductions_on_two_streams(gpu, restatement):
+    import torch
+    cases = [wl.linear_case(138 + i, 40000, 500, batch=64, with_bias=True) for i in range(2)]
+    put = lambda a: torch.from_numpy(a).cuda()  # noqa: E731
+    args = [[put(c[n]) for n in ("x", "bias32", "w")] for c in cases]
+    outs = [[torch.zeros((64, 500), dtype=torch.int32, device="cuda") for _ in range(2)] for _ in range(20)]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    api.set_batch(64)
+    try:
+        for pair in outs:
+            for (x, bias, w), out, s in zip(args, pair, streams):
+                api.set_stream(s.cuda_stream)
+                api.pulp_nn_linear_out_32(32, x, bias, out, w, 40000, 500)
+                assert api.last_kernel() == "igemm_tc_kernel"
+    finally:
+        api.set_stream(0)
+        api.set_batch(1)
+    torch.cuda.synchronize()
+    for i, c in enumerate(cases):
+        want = restatement.linear_out_32(c["x"], c["w"], bias32=c["bias32"])
+        for pair in outs:
+            same(pair[i].cpu().numpy(), want)
 
 
 # depthwise layers with one row of output, of which the plane kernel computes two or four
