@@ -499,7 +499,7 @@ bool launch_conv(Context &c, const ConvProblem &p)
       const double split = few == FewTiles::split ? igemm_split_estimate(c, p) : -1;
       auto ahead = [&](double t, double u) { return t >= 0 && 1.15 * t < u; };
       if (!ahead(gather, halo) && !ahead(igemm, halo) && !ahead(split, halo)) return launch_conv_halo_tc(c, p);
-      if (few == FewTiles::none) return gather >= 0 && gather < igemm ? launch_conv_gather_tc(c, p) : launch_igemm_tc(c, p);
+      if (few == FewTiles::none) return gather >= 0 && (igemm < 0 || gather < igemm) ? launch_conv_gather_tc(c, p) : launch_igemm_tc(c, p);
     }
   }
   switch (few) {

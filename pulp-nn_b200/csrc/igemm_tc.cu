@@ -857,6 +857,7 @@ bool igemm_tc_few_values(const ConvProblem &p)
 // its bytes 2.3 ns a KB, and the tile's drain 340 ns per 64 columns.
 double igemm_tc_spatial_estimate(const Context &c, const ConvProblem &p)
 {
+  if (!igemm_tc_supported(c, p)) return -1;
   bool few;
   const int sms = c.sm_count > 0 ? c.sm_count : 148, tiles = igemm_tc_tiles(c, p, &few), bkb = slab_bytes(p), bn = tile_columns(p);
   const double slabs = (p.ky * p.kx * p.Cin + bkb - 1) / bkb, rounds = tiles / sms + (tiles % sms != 0);

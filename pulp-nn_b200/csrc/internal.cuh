@@ -299,7 +299,7 @@ bool igemm_tc_few_values(const ConvProblem &p);
 // m-tiles x n-tiles that kernel cuts the problem into, and whether these are so few that it leaves the GPU idle over a
 // reduction of eight slabs or more
 int igemm_tc_tiles(const Context &c, const ConvProblem &p, bool *few);
-double igemm_tc_spatial_estimate(const Context &c, const ConvProblem &p);     // ns of a spatial kernel with whole rows
+double igemm_tc_spatial_estimate(const Context &c, const ConvProblem &p);     // ns of a spatial kernel with whole rows; -1 where it does not take the problem
 // the same GEMM computed by pairs of SMs (tcgen05 cta_group::2), for wide layers with a long reduction
 bool igemm_tc2_supported(const Context &c, const ConvProblem &p);
 bool launch_igemm_tc2(Context &c, const ConvProblem &p);
