@@ -3,6 +3,7 @@
 #include <cstdio>
 #include <cstring>
 #include <atomic>
+#include <new>
 
 #include "internal.cuh"
 
@@ -101,32 +102,51 @@ void *ctx_scratch(Context &c, size_t bytes)
   return c.scratch;
 }
 
+// For calls that a capture going on in another thread must not be ended by: memory that a thread allocates and frees for
+// itself is of no concern to a stream it does not use.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+Partials::~Partials()
+{
+  if (!done) return;
+  RelaxedCapture relaxed;
+  cudaEventSynchronize(done);
+  if (mem) cudaFree(mem);
+  cudaEventDestroy(done);
+}
+
 // Not under a stream capture: a graph would keep the address while the buffer grows, and be replayed on any stream.
 void *ctx_partials(Context &c, size_t bytes)
 {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(c.stream, &cap) != cudaSuccess) { cudaGetLastError(); return nullptr; }
   if (cap != cudaStreamCaptureStatusNone) return nullptr;
-  if (!c.partials_done && cudaEventCreateWithFlags(&c.partials_done, cudaEventDisableTiming) != cudaSuccess) {
-    cudaGetLastError();
-    c.partials_done = nullptr;
-    return nullptr;
-  }
-  if (bytes > c.partials_cap) {
-    cudaEventSynchronize(c.partials_done);
-    if (c.partials) cudaFree(c.partials);
-    c.partials = nullptr; c.partials_cap = 0;
+  Partials &p = c.partials;
+  if (bytes > p.cap) {
+    RelaxedCapture relaxed;
+    if (!p.done && cudaEventCreateWithFlags(&p.done, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      p.done = nullptr;
+      return nullptr;
+    }
+    cudaEventSynchronize(p.done);
+    if (p.mem) cudaFree(p.mem);
+    p.mem = nullptr; p.cap = 0;
     const size_t size = (bytes + (1u << 20) - 1) & ~(size_t)((1u << 20) - 1);
-    if (cudaMalloc(&c.partials, size) != cudaSuccess) { cudaGetLastError(); c.partials = nullptr; return nullptr; }
-    c.partials_cap = size;
+    if (cudaMalloc(&p.mem, size) != cudaSuccess) { cudaGetLastError(); p.mem = nullptr; return nullptr; }
+    p.cap = size;
   }
-  if (cudaStreamWaitEvent(c.stream, c.partials_done, 0) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-  return c.partials;
+  if (cudaStreamWaitEvent(c.stream, p.done, 0) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  return p.mem;
 }
 
 bool ctx_partials_done(Context &c)
 {
-  return cuda_ok(cudaEventRecord(c.partials_done, c.stream), "cudaEventRecord(partial sums)");
+  return cuda_ok(cudaEventRecord(c.partials.done, c.stream), "cudaEventRecord(partial sums)");
 }
 
 // device word that kernels with bounded waits report into (read by pulpnn_device_status)
@@ -226,10 +246,8 @@ int pulpnn_set_device(int device)
     for (auto &s : c.slots) { if (s.dev) cudaFree(s.dev); s.dev = nullptr; s.cap = 0; }
     if (c.scratch) cudaFree(c.scratch);
     c.scratch = nullptr; c.scratch_cap = 0;
-    if (c.partials) cudaFree(c.partials);
-    c.partials = nullptr; c.partials_cap = 0;
-    if (c.partials_done) cudaEventDestroy(c.partials_done);
-    c.partials_done = nullptr;
+    c.partials.~Partials();
+    new (&c.partials) Partials();
     if (c.status_word) cudaFree(c.status_word);
     c.status_word = nullptr;
     c.device = -1;

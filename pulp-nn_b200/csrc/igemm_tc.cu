@@ -998,7 +998,7 @@ bool launch_igemm_tc(Context &c, const ConvProblem &p, int slices)
     return launch_final(c, maps, g, bn, bkb, grid, tma_out);
   }
   const size_t part_bytes = (size_t)g.k_slices * g.M * g.N * sizeof(int);
-  int *partials = static_cast<int *>(requested ? ctx_scratch(c, part_bytes) : c.partials);
+  int *partials = static_cast<int *>(requested ? ctx_scratch(c, part_bytes) : c.partials.mem);
   if (!partials) return false;
   g.out = partials;
   g.vec_store = (g.N % 4 == 0);

@@ -182,6 +182,14 @@ struct PoolProblem {
 // ---------------------------------------------------------------------------------------------
 struct StageSlot { void *dev = nullptr; size_t cap = 0; };
 
+// Memory for the partial sums of the longest reductions, and when their latest reader was through with them; given back
+// when its thread ends.
+struct Partials {
+  void *mem = nullptr; size_t cap = 0;
+  cudaEvent_t done = nullptr;
+  ~Partials();
+};
+
 struct Context {
   int device = -1;
   cudaStream_t stream = nullptr;
@@ -196,9 +204,7 @@ struct Context {
   StageSlot slots[8];
   // device scratch owned by the context (split-K partial sums, status word)
   void *scratch = nullptr; size_t scratch_cap = 0;
-  // partial sums of the longest reductions, and when their latest reader was through with them
-  void *partials = nullptr; size_t partials_cap = 0;
-  cudaEvent_t partials_done = nullptr;
+  Partials partials;
   int *status_word = nullptr;     // device int, 0 = fine
   int sm_count = 0;
 };

@@ -154,6 +154,50 @@ def test_long_reductions_on_two_streams(gpu, restatement):
             same(pair[i].cpu().numpy(), want)
 
 
+def test_long_reduction_beside_a_capture_of_another_thread(gpu, restatement):
+    """A thread that gets memory for its sums, and gives it back at its end, while another one captures a graph."""
+    import threading
+
+    import torch
+    c = wl.linear_case(140, 40000, 500, batch=64, with_bias=True)
+    put = lambda a: torch.from_numpy(a).cuda()  # noqa: E731
+    x, w, bias = put(c["x"]), put(c["w"]), put(c["bias32"])
+    out, short = (torch.zeros((64, 500), dtype=torch.int32, device="cuda") for _ in range(2))
+    free, started, captured, took = [], threading.Event(), threading.Event(), []
+
+    def work():
+        torch.cuda.set_device(0)
+        api.set_device(0)
+        api.set_batch(64)
+        api.set_stream(stream)
+        api.pulp_nn_linear_out_32(32, x, bias, short, w, 4000, 500)      # what every thread allocates
+        api.synchronize()
+        started.set()
+        captured.wait(60)
+        api.pulp_nn_linear_out_32(32, x, bias, out, w, 40000, 500)
+        took.append(api.last_kernel())
+
+    for _ in range(8):
+        stream, side, g = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        out.zero_()
+        torch.cuda.synchronize()
+        started.clear()
+        captured.clear()
+        t = threading.Thread(target=work)
+        t.start()
+        assert started.wait(60)
+        with torch.cuda.graph(g, stream=side):
+            short.zero_()
+            captured.set()
+            t.join()
+        g.replay()
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert took == ["igemm_tc_kernel"] * 8 and not short.any()
+    assert free[1] - free[-1] < 8 << 20                  # the sums of one call alone are 2 MB in 16 slices each
+    same(out.cpu().numpy(), restatement.linear_out_32(c["x"], c["w"], bias32=c["bias32"]))
+
+
 # depthwise layers with one row of output, of which the plane kernel computes two or four
 @pytest.mark.parametrize("B,W,C,k,s,hwc,took", [
     (1, 1958, 128, 3, 2, True, "depthwise_hwc3x3_tma_kernel"), (15, 80, 32, 3, 1, False, "depthwise_chw3x3_tma_kernel"),
