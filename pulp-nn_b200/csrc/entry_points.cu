@@ -429,7 +429,9 @@ void add_entry(uint8_t *a, uint8_t *b, uint8_t *out, int m1, int m2, int out_shi
 //   -> 64 8.1 / 4.4 / 7.7 / 3.5, 14x14x64 -> 64 8.1 / 5.4 / 7.5 / 3.9, 28x28x128 -> 128 10.4 / 6.6 / 6.8 / 4.6, at batch 4
 //   7.4 / 9.1 / 8.2 / 5.3, 14x14x256 -> 256 at batch 8 14.3 / 11.1 / 9.1 / 7.2
 // Beyond 18000 terms the 16 slices of a split through memory (igemm_tc and a second kernel) leave the eight CTAs of a
-// cluster behind (not under a stream capture, whose graph would keep that memory's address): 1 x 17344 9.8 / 11.8, 1 x 60656 18.7 / 32.3, 9x9 58x12x512 -> 4 14.9 / 24.9 (12560 10.2 / 10.3).
+// cluster behind, but not under a stream capture, whose graph would keep the address of the sums. Calls one after the other,
+// slices / cluster: 1 x 18000 -> 4 10.8 / 12.3, -> 1000 13.2 / 13.4, 1 x 30000 -> 64 14.4 / 18.3, 1 x 60656 -> 4 19.9 / 32.5
+// (1.2 of these the event that orders streams), 9x9 58x12x512 -> 4 14.9 / 24.9 before that event (12560 terms 10.2 / 10.3).
 constexpr int LONG_REDUCTION = 18000;
 enum class FewTiles { none, rows, gather, split, slices };
 static FewTiles few_tiles_form(Context &c, const ConvProblem &p)
